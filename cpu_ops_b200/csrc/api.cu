@@ -1283,6 +1283,15 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       // well before four warps have drained the previous tile (about 1500 cycles per
       // 32-column chunk each): measured +10-15 % at K = 1024, nothing at K = 2048
       if (2 * (k_blocks / ch.slices) <= 3 * (ch.BN / 32) && ch.BN >= 128) epi_warps = 8;
+      // ... or when the chain holds a Gelu or Silu (about 20 instructions and two MUFU
+      // operations per element) and the k loop is not long enough for four warps to issue
+      // them behind it.  With bias + SiLU, four / eight warps: e4m3 2048 x 4096 x 2048 (16
+      // k-blocks) 48.8 / 40.3 us, 4096^3 (32) 92.1 / 89.0, 8192 x 2048 x 8192 (64) 150 / 159;
+      // e2m1 4096^3 (16) 78.5 / 64.2, 8192^3 (32) 319 / 307.
+      for (int t = 0; t < d->n_ops; ++t)
+        if ((d->ops[t].opcode == CPUOPS_B200_OP_GELU || d->ops[t].opcode == CPUOPS_B200_OP_SILU) &&
+            p.mode == kModeEpilogue && k_blocks <= 32 && ch.BN >= 128)
+          epi_warps = 8;
       if (env_switches().epi_warps == 8 || env_switches().epi_warps == 4) epi_warps = env_switches().epi_warps;
     }
     p.error = st.error_dev;
