@@ -149,67 +149,84 @@ int pick_tile_width(int Mk, int Nk, int k_blocks, bool is_mx, int sms, bool beta
 
 struct DecodePlan {
   bool use = false;
-  int BN = 32, tiles = 0, grid = 0, stages = 0, tile_aligned = 0, max_pieces = 1, tmem_cols = 128;
-  size_t partial_bytes = 0;
+  int BN = 32, tiles = 0, grid = 0, stages = 0, splits = 1, tmem_cols = 128;
   int smem = 0;
 };
 
-// Grid, ranges and buffers of a decode launch: Mk weight rows (128-row tiles), Nk <= 64
-// activation rows, k_blocks 128-byte k-blocks.  Every CTA takes an equal share of the
-// (tile, k-block) units; `never_split` (split_k_slices == 1) keeps whole tiles together.
-DecodePlan plan_decode(const DeviceState& st, int kind, int Mk, int Nk, int k_blocks, bool never_split) {
+// Clusters of `splits` CTAs of the decode kernel that can be resident at once (asked once per
+// device and size; a GPC's SMs are not a multiple of every size).
+int decode_clusters(DeviceState& st, int kind, int splits) {
+  int& known = st.decode_clusters[splits];
+  if (known < 0) {
+    cudaLaunchConfig_t probe = {};
+    probe.gridDim = dim3(static_cast<unsigned>(splits * st.sm_count));
+    probe.blockDim = dim3(kDecodeThreads);
+    probe.dynamicSmemBytes = static_cast<size_t>(120 * 1024);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    probe.attrs = attr;
+    probe.numAttrs = 1;
+    int n = 0;
+    const cudaError_t e = kind == kKindMxf4
+                              ? cudaOccupancyMaxActiveClusters(&n, decode_mx_kernel<kKindMxf4>, &probe)
+                              : cudaOccupancyMaxActiveClusters(&n, decode_mx_kernel<kKindMxf8>, &probe);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    known = n;
+  }
+  return known;
+}
+
+// Grid, split and buffers of a decode launch: Mk weight rows (128-row tiles), Nk <= 64
+// activation rows, k_blocks 128-byte k-blocks.  `never_split` (split_k_slices == 1) keeps
+// whole tiles.
+DecodePlan plan_decode(DeviceState& st, int kind, int Mk, int Nk, int k_blocks, bool never_split) {
   DecodePlan dp;
   dp.use = true;
   dp.BN = Nk <= 32 ? 32 : 64;
   dp.tiles = (Mk + kTileM - 1) / kTileM;
   const int ka = kind == kKindMxf4 ? 2 : 1;
   const int per_stage = decode_stage_bytes(Nk) + 2 * ka * 512;
-  // One CTA per SM with the deepest ring the shared memory allows: the stream needs the
-  // bytes in flight (two smaller CTAs per SM measured slower).
-  int ctas_per_sm = 1;
-  if (env_switches().decode_ctas_per_sm > 0) ctas_per_sm = env_switches().decode_ctas_per_sm;
-  const int64_t units = static_cast<int64_t>(dp.tiles) * k_blocks;
-  const int cap = st.sms() * ctas_per_sm;
-  int grid;
-  if (never_split || 4 * dp.tiles >= cap) {
-    // whole tiles per CTA: no partial sums.  (Measured on 112 tiles: cutting k to feed all
-    // 148 SMs does not shorten the stream, and the reduction through L2 costs 4 us.)  k is
-    // only cut when the tiles are too few to keep even a quarter of the SMs busy.
-    grid = std::min(dp.tiles, cap);
-    dp.tile_aligned = 1;
-  } else {
-    grid = static_cast<int>(std::min<int64_t>(cap, std::max<int64_t>(1, units / 4)));  // >= 4 units per CTA
-    if (dp.tiles >= grid && dp.tiles % grid == 0) dp.tile_aligned = 1;
+  const int cap = st.sms();
+  dp.grid = std::min(dp.tiles, cap);
+  if (!never_split) {
+    // Fewer tiles than SMs: several CTAs per tile, each with at least three k-blocks, on at
+    // most all but 16 SMs: while some SMs are free the next call's CTAs become resident early
+    // and only then is their prologue hidden (74 tiles of 32 k-blocks: 74 CTAs 12.3 us, 148
+    // CTAs 13.3; clusters of 8 are slower than of 6: 8 tiles 5.4 / 4.9 us).  Cutting in
+    // two saves less than the exchange costs unless the halves are long (56 tiles: of 16
+    // k-blocks 7.4 -> 7.7 us, of 32 11.3 -> 10.1; 32 tiles of 16 in four 7.1 -> 6.9, of 32
+    // 11.2 -> 8.7, of 112 in four 32.5 -> 14.8).
+    int want = std::min({kDecodeMaxSplits, (cap - 16) / std::max(1, dp.tiles), k_blocks / 3});
+    if (want == 2 && k_blocks < 24) want = 1;
+    if (env_switches().decode_splits > 0) want = std::min(env_switches().decode_splits, k_blocks);
+    for (int s = want; s >= 2; --s) {
+      if (decode_clusters(st, kind, s) < dp.tiles) continue;
+      dp.splits = s;
+      dp.grid = dp.tiles * s;
+      break;
+    }
   }
-  if (env_switches().decode_grid > 0 && !never_split) {
-    grid = static_cast<int>(std::min<int64_t>(env_switches().decode_grid, units));
-    dp.tile_aligned = (dp.tiles % grid == 0) ? 1 : 0;
-  }
-  dp.grid = grid;
-  const int budget = st.smem_optin / ctas_per_sm - (ctas_per_sm > 1 ? 1024 : 0);
-  int stages = (budget - 1024 - decode_staging_bytes(dp.BN) - kDecodeBarrierBytes) / per_stage;
-  stages = std::min({stages, kDecodeMaxStages, static_cast<int>(std::max<int64_t>(2, (units + grid - 1) / grid))});
+  const int units = dp.splits > 1 ? (k_blocks + dp.splits - 1) / dp.splits
+                                  : (dp.tiles + dp.grid - 1) / dp.grid * k_blocks;  // most per CTA
+  // the deepest ring the shared memory allows: the stream needs the bytes in flight
+  int stages = (st.smem_optin - 1024 - decode_staging_bytes(dp.BN) - decode_reduce_bytes(Nk, dp.splits) - kDecodeBarrierBytes) /
+               per_stage;
+  stages = std::min({stages, kDecodeMaxStages, std::max(2, units)});
   if (env_switches().decode_stages > 0) stages = std::min(stages, env_switches().decode_stages);
   dp.stages = std::max(2, stages);
-  dp.smem = decode_smem_bytes(Nk, dp.BN, dp.stages, 2 * ka);
-  // one CTA per SM must not be joined by a second one that would queue behind its TMEM
-  if (ctas_per_sm == 1) dp.smem = std::max(dp.smem, 120 * 1024);
+  dp.smem = decode_smem_bytes(Nk, dp.BN, dp.stages, 2 * ka, dp.splits);
+  // one CTA per SM must not be joined by a second one of the same launch
+  dp.smem = std::max(dp.smem, 120 * 1024);
   const int sf_cols = 4 * 2 * ka;
   int cols = 2 * dp.BN + kDecodeSfSlots * sf_cols;
   dp.tmem_cols = 32;
   while (dp.tmem_cols < cols) dp.tmem_cols *= 2;
-  if (!dp.tile_aligned) {
-    DecodeParams q;
-    memset(&q, 0, sizeof(q));
-    q.tiles = dp.tiles;
-    q.k_blocks = k_blocks;
-    for (int t = 0; t < dp.tiles; ++t) {
-      const int first = decode_cta_of_unit(q, static_cast<int64_t>(t) * k_blocks, grid);
-      const int last = decode_cta_of_unit(q, static_cast<int64_t>(t + 1) * k_blocks - 1, grid);
-      dp.max_pieces = std::max(dp.max_pieces, last - first + 1);
-    }
-    dp.partial_bytes = static_cast<size_t>(dp.tiles) * dp.max_pieces * dp.BN * kTileM * 4;
-  }
   return dp;
 }
 
@@ -416,7 +433,6 @@ CPUOPS_B200_API int cpuops_b200_stream_status(void* stream) {
     set_error("device-side bounded wait timed out (code %d)", *st->error_host);
     *st->error_host = 0;
     CUDA_TRY(cudaMemsetAsync(st->error_dev, 0, sizeof(int32_t), s));
-    reset_counters(*st, s);
     CUDA_TRY(cudaStreamSynchronize(s));
     return CPUOPS_B200_STATUS_DEVICE_TIMEOUT;
   }
@@ -582,7 +598,6 @@ static int run_host_row_panels(const cpuops_b200_gemm_desc* d, DeviceState& st, 
     set_error("device-side bounded wait timed out (code %d)", *st.error_host);
     *st.error_host = 0;
     cudaMemsetAsync(st.error_dev, 0, sizeof(int32_t), stream);
-    reset_counters(st, stream);
     cudaStreamSynchronize(stream);
     return CPUOPS_B200_STATUS_DEVICE_TIMEOUT;
   }
@@ -798,8 +813,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   // forced tile width or slice count keeps the general kernel, whose plan those describe.
   DecodePlan dp;
   if (k > 0 && is_mx && !mixed && ch.swap && m <= 64 && d->tile_n == 0 && d->split_k_slices <= 1 &&
-      !(d->flags & (CPUOPS_B200_FLAG_PAIR_ON | CPUOPS_B200_FLAG_PAIR_OFF)) && !env_switches().no_decode &&
-      (n + kTileM - 1) / kTileM <= kDecodeMaxTiles) {
+      !(d->flags & (CPUOPS_B200_FLAG_PAIR_ON | CPUOPS_B200_FLAG_PAIR_OFF)) && !env_switches().no_decode) {
     auto scales_ok = [](const void* ptr, bool on_device, int ld, int rows) {
       return (!on_device || (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0) && (rows <= 1 || ld % 16 == 0);
     };
@@ -814,7 +828,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   Plan plan;
   const int64_t c_outer = c_rm ? m : n, c_inner = c_rm ? n : m;
   size_t off_a = 0, off_b = 0, off_sa = 0, off_sb = 0, off_c = 0, off_d = 0, off_sfa = 0, off_sfb = 0,
-         off_ws = 0, off_partial = 0, off_ops[CPUOPS_B200_MAX_OPS] = {0};
+         off_ws = 0, off_ops[CPUOPS_B200_MAX_OPS] = {0};
   int64_t a_pitch_dev = A.pitch, b_pitch_dev = B.pitch;
   bool a_repack = false, b_repack = false;
   const bool a_mask = fp4_a && (k & 1), b_mask = fp4_b && (k & 1);
@@ -868,9 +882,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   if (k > 0) {
     Mk = ch.swap ? n : m;
     Nk = ch.swap ? m : n;
-    if (dp.use) {
-      if (dp.partial_bytes) off_partial = plan.take(dp.partial_bytes);
-    } else if (is_mx) {
+    if (is_mx && !dp.use) {
       bps = fp4_pair ? 8 : 4;
       // a pair always reads the scales of both of its 128-row halves
       sfa_bytes = cpuops_b200_scale_layout_bytes(ch.pair ? static_cast<int>(align_up(Mk, 256)) : Mk, k,
@@ -1027,8 +1039,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     q.k_blocks = k_blocks;
     q.BN = dp.BN;
     q.stages = dp.stages;
-    q.tile_aligned = dp.tile_aligned;
-    q.max_pieces = dp.max_pieces;
+    q.splits = dp.splits;
     q.tmem_cols = dp.tmem_cols;
     if (kind == kKindMxf4) {
       q.idesc = make_idesc_block_scaled(1u, 1u, kTileM, dp.BN);  // e2m1 x e2m1
@@ -1038,8 +1049,6 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     }
     q.wait_budget_us = g_wait_budget_us.load();
     q.epi = epi;
-    q.partial = reinterpret_cast<float*>(wsp + off_partial);
-    if (int rc = ensure_counters(st, stream, &q.counters)) return rc;
     q.error = st.error_dev;
 #ifdef CPUOPS_B200_INSTRUMENT
     if (env_switches().clk) {
@@ -1070,13 +1079,17 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     cfg.blockDim = dim3(kDecodeThreads);
     cfg.dynamicSmemBytes = static_cast<size_t>(dp.smem);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     // The kernel may start while the kernel before it in the stream is finishing; every
     // role waits for that kernel before it touches memory (see decode_kernel.cuh).
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(dp.splits);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dp.splits > 1 ? 2 : 1;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     const bool profile = g_profile.load();
     if (profile) {
@@ -1087,7 +1100,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     g_last_plan = cpuops_b200_plan{};
     g_last_plan.swapped = 1;
     g_last_plan.tile_n = dp.BN;
-    g_last_plan.slices = dp.max_pieces;
+    g_last_plan.slices = dp.splits;
     g_last_plan.stages = dp.stages;
     g_last_plan.grid = dp.grid;
     g_last_plan.epilogue_warps = 4;
@@ -1450,7 +1463,6 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     set_error("device-side bounded wait timed out (code %d)", *st.error_host);
     *st.error_host = 0;
     cudaMemsetAsync(st.error_dev, 0, sizeof(int32_t), stream);
-    reset_counters(st, stream);
     cudaStreamSynchronize(stream);
     return CPUOPS_B200_STATUS_DEVICE_TIMEOUT;
   }

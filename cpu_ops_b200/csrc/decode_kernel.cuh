@@ -15,29 +15,32 @@
 //     memory, ahead of the MMAs.  (Measured: a 16-byte wide TMA box per stage instead costs
 //     the TMA unit as much time as the 128-byte wide operand box -- it works row by row --
 //     and halved the stream.)
-//   * The work is cut into (tile, k-block) units and every CTA takes an equal, contiguous
-//     range of them, so all SMs stream for the same time whatever the tile count.  A CTA's
-//     range meets at most a few tiles; a piece that covers a tile's whole k extent goes
-//     through the epilogue directly, the others are written as partial sums and the warp
-//     that arrives last for a (tile, lane quarter) adds the pieces in ascending k order --
-//     a fixed order, so results do not depend on which CTA finished first.
+//   * A CTA takes whole tiles while there are enough of them to fill the SMs.  When there are
+//     fewer, a cluster of 2 to 6 CTAs shares each tile, every CTA a contiguous part of k: the
+//     partial accumulators meet in distributed shared memory (st.async straight into the
+//     owner's buffer, its barrier counting the bytes), and each owner adds the pieces of its
+//     part in ascending k order - a fixed order, so results do not depend on which CTA
+//     finished first.  The cut of a tile never leaves the chip and needs no workspace.
 //   * Launched with programmatic stream serialization: a CTA may become resident and set up
 //     its barriers and tensor memory while the kernel before this one in the stream is
 //     still finishing; every role then waits (griddepcontrol.wait) before it reads or
 //     writes global memory.
 //
-// Where the time of one call goes (14336 x 4096 fp4 weights, m = 8, calls back to back,
-// time stamps of every role in an instrumented build): 10.1 us per call against 14.6 us for
-// the general kernel with its separate re-layout launch; of these the HBM stream itself is
-// 5.0 us (5.9 TB/s), the latency of the first bytes after the wait 1.3 us, the tail after
-// the last byte 1.3 us and the gap between a kernel's last CTA leaving and its successor
-// passing the wait 1.3 us.  Tried and not kept, each measured on the same loop: cutting k
-// so that all 148 SMs stream (the reduction through L2 costs 4 us, the stream gets no
-// shorter); asking W into L2 ahead of the wait with prefetch instructions, 256-byte fill
-// hints or TMA prefetch boxes (no gain; the TMA form costs the TMA unit as much as the
-// loads); two smaller CTAs per SM so that the next call's CTAs sit beside this call's,
-// with or without loading their first ring of W before the wait (the shallower ring
-// slows the stream by what the overlap saves).
+// Where the time of one call goes (14336 x 4096 fp4 weights, m = 1, calls back to back over
+// weights that are not in L2: 8.4 us per call; time stamps of every role in an instrumented
+// build): the HBM stream itself 5.0 us (5.9 TB/s), the latency of the first bytes after the
+// wait 1.3 us, the tail after the last byte and the gap between a kernel's last CTA leaving
+// and its successor passing the wait 1 us each.  Cutting a tile's k over a cluster instead of
+// through partial sums in global memory (a chain of dependent L2 round trips of about 4 us):
+// e4m3 m = 32, 4096 weight rows x k = 14336 21.2 -> 14.4 us, x k = 4096 15.5 -> 8.9 us;
+// e2m1 m = 1, 4096 x 14336 16.1 -> 9.8 us; 1024 x 4096 8.7 -> 5.1 us.
+//
+// Tried and not kept, each measured on the same loop: asking W into L2 ahead of the wait,
+// with untiled bulk prefetches of the CTA's whole share (8.4 -> 10.3 us: they queue in the
+// same unit as the loads), with prefetch instructions for the first 2, 4, 8 or 12 k-blocks
+// (within 0.3 us either way), with 256-byte fill hints or TMA prefetch boxes; two smaller
+// CTAs per SM so that the next call's CTAs sit beside this call's (8.4 -> 9.3 us: the
+// shallower ring slows the stream by what the overlap saves), with and without prefetch.
 //
 // Roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer (owns tensor memory), warps
 // 2-5 scale writers (thread = tile row), warps 6-9 epilogue (one TMEM lane quarter each).
@@ -68,14 +71,11 @@ struct DecodeParams {
   int32_t tiles, k_blocks;   // 128-row tiles of W, 128-byte k-blocks
   int32_t BN;                // 32 or 64
   int32_t stages;
-  int32_t tile_aligned;      // 1: CTA ranges end on tile boundaries (no partial sums)
-  int32_t max_pieces;        // most pieces any tile is cut into (partial-sum slots per tile)
+  int32_t splits;            // CTAs (one cluster) that share a tile's k; 1: whole tiles per CTA
   int32_t tmem_cols;         // power of two >= 2 * BN + kDecodeSfSlots * scale columns per unit
   uint32_t idesc;
   uint32_t wait_budget_us;   // budget of every bounded wait
   EpilogueParams epi;
-  float* partial;            // [tile][piece][BN columns][128 rows]
-  int32_t* counters;         // [tile][4 lane quarters], zero between launches
   int32_t* error;
 #ifdef CPUOPS_B200_INSTRUMENT
   unsigned long long* clk;   // instrumented build: min / max over CTAs of role time stamps (ns)
@@ -104,40 +104,40 @@ __host__ __device__ inline int decode_x_bytes(int Nk) { return (Nk * 128 + 1023)
 __host__ __device__ inline int decode_stage_bytes(int Nk) { return kTileM * 128 + decode_x_bytes(Nk); }
 __host__ __device__ inline int decode_staging_bytes(int BN) { return kDecodeFetchAhead * (kTileM + BN) * 16; }
 constexpr int kDecodeBarrierBytes = 512;
-__host__ __device__ inline int decode_smem_bytes(int Nk, int BN, int stages, int atoms_per_unit) {
+// The reduction works in units of one lane quarter (32 rows) x 16 columns: 2 KB per source CTA.
+// Unit u belongs to CTA u % splits of the cluster, as its slot u / splits.
+constexpr int kDecodeUnitBytes = 32 * 16 * 4;
+__host__ __device__ inline int decode_reduce_units(int Nk) { return 4 * ((Nk + 15) / 16); }
+__host__ __device__ inline int decode_reduce_bytes(int Nk, int splits) {
+  if (splits <= 1) return 0;
+  return (decode_reduce_units(Nk) + splits - 1) / splits * splits * kDecodeUnitBytes;
+}
+constexpr int kDecodeMaxSplits = 6;
+constexpr int kDecodeMaxSlots = 8;  // 16 units over at least 2 CTAs
+__host__ __device__ inline int decode_smem_bytes(int Nk, int BN, int stages, int atoms_per_unit, int splits) {
   return 1024 + stages * (decode_stage_bytes(Nk) + atoms_per_unit * 512) + decode_staging_bytes(BN) +
-         kDecodeBarrierBytes;
+         decode_reduce_bytes(Nk, splits) + kDecodeBarrierBytes;
 }
 
-// Units [u0, u1) of CTA `c` out of `G`.
-__host__ __device__ inline int64_t decode_range_start(const DecodeParams& p, int c, int G) {
-  if (p.tile_aligned) return (static_cast<int64_t>(c) * p.tiles / G) * p.k_blocks;
-  return static_cast<int64_t>(c) * p.tiles * p.k_blocks / G;
-}
-// CTA whose range holds unit u (ranges not tile aligned).
-__host__ __device__ inline int decode_cta_of_unit(const DecodeParams& p, int64_t u, int G) {
-  const int64_t U = static_cast<int64_t>(p.tiles) * p.k_blocks;
-  return static_cast<int>(((u + 1) * G - 1) / U);
-}
-
-// alpha * acc + beta * C, the chain ops, and the store of one 32-column chunk of one row.
-__device__ __forceinline__ void decode_store_chunk(const EpilogueParams& e, uint32_t (&r)[32], int krow,
+// alpha * acc + beta * C, the chain ops, and the store of one N-column chunk of one row.
+template <int N>
+__device__ __forceinline__ void decode_store_chunk(const EpilogueParams& e, uint32_t (&r)[N], int krow,
                                                    int kcol0, int ncols) {
-  uint32_t src[32];
+  uint32_t src[N];
   if (e.beta_nonzero) {
     const uint32_t* c = static_cast<const uint32_t*>(e.C) + (krow * e.c_sr + kcol0 * e.c_sc);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) src[i] = i < ncols ? c[i * e.c_sc] : 0u;
+    for (int i = 0; i < N; ++i) src[i] = i < ncols ? c[i * e.c_sc] : 0u;
   } else {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) src[i] = 0u;
+    for (int i = 0; i < N; ++i) src[i] = 0u;
   }
 #pragma unroll
-  for (int i = 0; i < 32; ++i) r[i] = linear_combine_bits<false>(e, r[i], src[i]);
-  for (int t = 0; t < e.n_ops; ++t) apply_op_chunk<false>(e.ops[t], r, krow, kcol0, ncols);
+  for (int i = 0; i < N; ++i) r[i] = linear_combine_bits<false>(e, r[i], src[i]);
+  for (int t = 0; t < e.n_ops; ++t) apply_op_chunk<false, N>(e.ops[t], r, krow, kcol0, ncols);
   uint32_t* d = static_cast<uint32_t*>(e.D) + (krow * e.d_sr + kcol0 * e.d_sc);
 #pragma unroll
-  for (int i = 0; i < 32; ++i)
+  for (int i = 0; i < N; ++i)
     if (i < ncols) d[i * e.d_sc] = r[i];
 }
 
@@ -169,24 +169,29 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
   const uint32_t atom_bytes = 2u * kKa * 512u;
   const uint32_t atom_base = smem_base + stages * stage_bytes;
   const uint32_t staging_base = atom_base + stages * atom_bytes;
-  const uint32_t bar_base = staging_base + static_cast<uint32_t>(decode_staging_bytes(BN));
+  const uint32_t red_base = staging_base + static_cast<uint32_t>(decode_staging_bytes(BN));
+  const uint32_t bar_base = red_base + static_cast<uint32_t>(decode_reduce_bytes(p.Nk, p.splits));
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (kDecodeMaxStages + s); };
   auto acc_full_bar = [&](int b) { return bar_base + 8u * (2 * kDecodeMaxStages + b); };
   auto acc_empty_bar = [&](int b) { return bar_base + 8u * (2 * kDecodeMaxStages + 2 + b); };
   const uint32_t drain_bar = bar_base + 8u * (2 * kDecodeMaxStages + 4);
-  constexpr int kBarriers = 2 * kDecodeMaxStages + 5;
+  auto red_bar = [&](int slot) { return bar_base + 8u * (2 * kDecodeMaxStages + 5 + slot); };
+  constexpr int kBarriers = 2 * kDecodeMaxStages + 5 + kDecodeMaxSlots;
   static_assert(8 * kBarriers + 8 <= kDecodeBarrierBytes, "barrier region too small");
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + (bar_base - smem_base) + 8 * kBarriers);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint64_t budget_ns = static_cast<uint64_t>(p.wait_budget_us) * 1000ull;
 
-  // This CTA's units.
-  const int G = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
-  const int KB = p.k_blocks;
-  const int64_t u0 = decode_range_start(p, cta, G), u1 = decode_range_start(p, cta + 1, G);
-  const int n_units = static_cast<int>(u1 - u0);
-  const int tile0 = static_cast<int>(u0 / KB), kb0 = static_cast<int>(u0 - static_cast<int64_t>(tile0) * KB);
+  // This CTA's units: its cluster's tiles x its part of k.
+  const int splits = p.splits;
+  const int rank = splits > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
+  const int groups = static_cast<int>(gridDim.x) / splits, group = static_cast<int>(blockIdx.x) / splits;
+  const int tile0 = static_cast<int>(static_cast<int64_t>(group) * p.tiles / groups);
+  const int tile1 = static_cast<int>(static_cast<int64_t>(group + 1) * p.tiles / groups);
+  const int kb0 = static_cast<int>(static_cast<int64_t>(rank) * p.k_blocks / splits);
+  const int kb1 = static_cast<int>(static_cast<int64_t>(rank + 1) * p.k_blocks / splits);
+  const int n_units = (tile1 - tile0) * (kb1 - kb0);
 
   if (warp == 2) {
     for (int i = lane; i < kBarriers; i += 32) {
@@ -201,6 +206,10 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
     }
     if (lane == 0) *abort_flag = 0;
     fence_mbar_init();
+    __syncwarp();
+    // reduction slots: all pieces of this CTA's units, in bytes
+    if (splits > 1 && lane < kDecodeMaxSlots && rank + lane * splits < decode_reduce_units(p.Nk))
+      mbar_expect_tx(red_bar(lane), static_cast<uint32_t>(splits * kDecodeUnitBytes));
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), static_cast<uint32_t>(p.tmem_cols));
@@ -211,6 +220,9 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
     prefetch_tensormap(&tmX);
   }
   tc_fence_before_sync();
+  // (the epilogue warps wait for this arrival of every CTA of the cluster before they send
+  // anything: the reduction barriers are armed by then)
+  if (splits > 1) cluster_arrive();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
@@ -244,7 +256,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       mbar_expect_tx_p(full_bar(s), tx_bytes, el);
       issue_w(s, tile, kb);
       issue_x(s, kb);
-      if (++kb == KB) { kb = 0; ++tile; }
+      if (++kb == kb1) { kb = kb0; ++tile; }
       if (++s == stages) { s = 0; ph ^= 1u; }
     }
     DECODE_STAMP(p, 3, el);
@@ -276,13 +288,12 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       id3 = id1;
     }
     const uint32_t sf_t0 = tmem_base + 2u * static_cast<uint32_t>(BN);
-    int s = 0, buf = 0, kb = kb0, sf_q = 0;
+    int s = 0, buf = 0, sf_q = 0;
     uint32_t ph = 0, acc_ph = 0;
     bool ok = true;
     int i = 0;
     while (i < n_units && ok) {
-      // one piece: the units of this range that belong to one tile
-      const int piece_units = min(KB - kb, n_units - i);
+      const int piece_units = kb1 - kb0;  // one tile
       if (!__all_sync(kAll, mbar_wait_bounded(acc_empty_bar(buf), acc_ph ^ 1u, abort_flag, budget_ns))) {
         if (el) {
           atomicCAS(p.error, 0, kErrMmaWaitAcc);
@@ -333,7 +344,6 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       tc_commit_g<false>(acc_full_bar(buf), el);
       if (++buf == 2) { buf = 0; acc_ph ^= 1u; }
       i += piece_units;
-      kb = 0;
     }
     // nothing may still be executing when tensor memory is released
     tc_commit_g<false>(drain_bar, el);
@@ -376,9 +386,9 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
                        : "memory");
         }
         const int next_kb = (f_kb | (kUnitsPerChunk - 1)) + 1;
-        if (next_kb >= KB) {
-          f_i += KB - f_kb;
-          f_kb = 0;
+        if (next_kb >= kb1) {
+          f_i += kb1 - f_kb;
+          f_kb = kb0;
           ++f_tile;
         } else {
           f_i += next_kb - f_kb;
@@ -393,8 +403,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
     uint4 cur_w = make_uint4(0, 0, 0, 0), cur_x = make_uint4(0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
     bool alive = true;
     while (i < n_units && alive) {
-      // one chunk: the units that share this 16-byte fetch (up to the tile's and the range's end)
-      const int in_chunk = min(min(kUnitsPerChunk - (kb & (kUnitsPerChunk - 1)), KB - kb), n_units - i);
+      // one chunk: the units that share this 16-byte fetch (up to the end of this CTA's part of k)
+      const int in_chunk = min(kUnitsPerChunk - (kb & (kUnitsPerChunk - 1)), kb1 - kb);
       asm volatile("cp.async.wait_group %0;" ::"n"(kDecodeFetchAhead - 1) : "memory");
       asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                    : "=r"(cur_w.x), "=r"(cur_w.y), "=r"(cur_w.z), "=r"(cur_w.w)
@@ -441,108 +451,133 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       ph = ph2;
       i += in_chunk;
       kb += in_chunk;
-      if (kb == KB) kb = 0;
+      if (kb == kb1) kb = kb0;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else {
     // -------------------------------- epilogue --------------------------------
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // before C is read, D / partial sums written
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // before C is read, D written
     const int q = warp & 3;  // the TMEM lane quarter this warp can read
-    const int nchunks = BN / 32;
+    const int nchunks = (p.Nk + 15) / 16;
     const EpilogueParams& e = p.epi;
     warm_epilogue_params(e);
-    asm volatile("" ::"r"(p.Mk ^ p.Nk ^ p.max_pieces), "l"(p.partial), "l"(p.counters));
-    int buf = 0, kb = kb0, tile = tile0, i = 0;
+    int buf = 0;
     uint32_t acc_ph = 0;
-    while (i < n_units) {
-      const int piece_units = min(KB - kb, n_units - i);
-      const bool whole = kb == 0 && piece_units == KB;
+    bool alive = true;
+    if (splits > 1) cluster_wait();
+    for (int tile = tile0; tile < tile1; ++tile) {
       const bool got = mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
       if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) {
           atomicCAS(p.error, 0, kErrEpilogueWait);
           *abort_flag = 1;
         }
+        alive = false;
         break;
       }
       tc_fence_after_sync();
-      if (i + piece_units == n_units) DECODE_STAMP(p, 6, warp == 6 && lane == 0);
+      if (tile + 1 == tile1) DECODE_STAMP(p, 6, warp == 6 && lane == 0);
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
-      const int row_in_tile = q * 32 + lane;
-      const int krow = tile * kTileM + row_in_tile;
-      int pieces = 1, piece = 0;
-      if (!whole) {
-        const int first = decode_cta_of_unit(p, static_cast<int64_t>(tile) * KB, G);
-        const int last = decode_cta_of_unit(p, static_cast<int64_t>(tile + 1) * KB - 1, G);
-        pieces = last - first + 1;
-        piece = cta - first;
-      }
-      float* my_partial = p.partial + ((static_cast<int64_t>(tile) * p.max_pieces + piece) * BN) * kTileM + row_in_tile;
-      for (int c = 0; c < nchunks; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + static_cast<uint32_t>(c * 32), r);
-        tmem_ld_wait();
-        if (i + piece_units == n_units && c == 0) DECODE_STAMP(p, 8, warp == 6 && lane == 0);
-        if (c + 1 == nchunks) {
-          // the accumulator is in registers: hand the buffer back to the MMA warp
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(acc_empty_bar(buf));
-        }
-        if (i + piece_units == n_units && c == 0) DECODE_STAMP(p, 9, warp == 6 && lane == 0);
-        const int kcol0 = c * 32, ncols = min(32, p.Nk - kcol0);
-        if (whole) {
-          if (krow < p.Mk && ncols > 0) decode_store_chunk(e, r, krow, kcol0, ncols);
-          if (i + piece_units == n_units && c == 0) DECODE_STAMP(p, 10, warp == 6 && lane == 0);
-        } else {
-          // raw partial sums, column by column: a warp writes 128 contiguous bytes per column
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < ncols) __stcg(my_partial + static_cast<int64_t>(kcol0 + j) * kTileM, __uint_as_float(r[j]));
-        }
-      }
-      if (!whole) {
-        // Last arriver of this (tile, lane quarter) adds the pieces in ascending k order.
-        __threadfence();
+      const int krow = tile * kTileM + q * 32 + lane;
+      // the accumulator is in registers: hand the buffer back to the MMA warp
+      auto hand_back = [&]() {
+        tc_fence_before_sync();
         __syncwarp();
-        int old = 0;
-        if (lane == 0) old = atomicAdd(p.counters + tile * 4 + q, 1);
-        old = __shfl_sync(0xffffffffu, old, 0);
-        if (old == pieces - 1) {
-          __threadfence();
-          const float* base = p.partial + (static_cast<int64_t>(tile) * p.max_pieces * BN) * kTileM + row_in_tile;
-          for (int c = 0; c < nchunks; ++c) {
-            const int kcol0 = c * 32, ncols = min(32, p.Nk - kcol0);
-            if (ncols <= 0) break;
-            // piece by piece, all columns of a piece in flight together (one L2 round trip
-            // per piece, not per element); per element the order is still piece 0, 1, 2, ...
-            float acc[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              acc[j] = j < ncols ? __ldcg(base + static_cast<int64_t>(kcol0 + j) * kTileM) : 0.0f;
-            for (int pi = 1; pi < pieces; ++pi) {
-              const float* pb = base + static_cast<int64_t>(pi) * BN * kTileM;
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (j < ncols) acc[j] = __fadd_rn(acc[j], __ldcg(pb + static_cast<int64_t>(kcol0 + j) * kTileM));
-            }
-            uint32_t r[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(acc[j]);
-            if (krow < p.Mk) decode_store_chunk(e, r, krow, kcol0, ncols);
-          }
-          if (lane == 0) p.counters[tile * 4 + q] = 0;  // ready for the next launch
+        if (lane == 0) mbar_arrive(acc_empty_bar(buf));
+      };
+      if (splits == 1 && p.Nk > 16) {
+        for (int c = 0; c < p.Nk; c += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + static_cast<uint32_t>(c), r);
+          tmem_ld_wait();
+          if (c + 32 >= p.Nk) hand_back();
+          if (krow < p.Mk) decode_store_chunk<32>(e, r, krow, c, min(32, p.Nk - c));
         }
+      } else if (splits == 1) {
+        uint32_t r[16];
+        tmem_ld_32x16(taddr, r);
+        tmem_ld_wait();
+        if (tile + 1 == tile1) DECODE_STAMP(p, 8, warp == 6 && lane == 0);
+        hand_back();
+        if (krow < p.Mk) decode_store_chunk<16>(e, r, krow, 0, p.Nk);
+        if (tile + 1 == tile1) DECODE_STAMP(p, 10, warp == 6 && lane == 0);
+      } else {
+        for (int c = 0; c < nchunks; ++c) {
+          uint32_t r[16];
+          tmem_ld_32x16(taddr + static_cast<uint32_t>(c * 16), r);
+          tmem_ld_wait();
+          // this lane's 64 bytes of the unit, 16-byte pieces XOR-swizzled over pairs of lanes
+          // (rows are 64 bytes apart: without it every other lane would meet the same banks)
+          const int u = q + 4 * c, owner = u % splits, slot = u / splits;
+          const uint32_t dst = map_to_cta(
+              red_base + static_cast<uint32_t>((slot * splits + rank) * kDecodeUnitBytes + lane * 64),
+              static_cast<uint32_t>(owner));
+          const uint32_t bar = map_to_cta(red_bar(slot), static_cast<uint32_t>(owner));
+          const uint32_t swz = static_cast<uint32_t>(lane >> 1) & 3u;
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j)
+            st_async_v4(dst + ((j ^ swz) << 4), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], bar);
+        }
+        hand_back();
       }
       if (++buf == 2) { buf = 0; acc_ph ^= 1u; }
-      i += piece_units;
-      kb = 0;
-      ++tile;
+    }
+    if (splits > 1) cluster_arrive();  // nothing more leaves this warp for another CTA
+    if (splits > 1 && alive) {
+      // the units this CTA owns: the pieces added in ascending k order, then the epilogue
+      const int units = decode_reduce_units(p.Nk);
+      for (int slot = warp - 6; rank + slot * splits < units; slot += 4) {
+        const bool got = mbar_wait_bounded(red_bar(slot), 0, abort_flag, budget_ns);
+        if (!__all_sync(0xffffffffu, got)) {
+          if (lane == 0) {
+            atomicCAS(p.error, 0, kErrEpilogueWait);
+            *abort_flag = 1;
+          }
+          break;
+        }
+        const int u = rank + slot * splits;
+        const uint32_t swz = static_cast<uint32_t>(lane >> 1) & 3u;
+        uint32_t src = red_base + static_cast<uint32_t>(slot * splits * kDecodeUnitBytes + lane * 64);
+        float acc[16];
+        for (int pc = 0; pc < splits; ++pc, src += kDecodeUnitBytes) {
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j) {
+            float4 v;
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "r"(src + ((j ^ swz) << 4)));
+            acc[4 * j] = pc == 0 ? v.x : __fadd_rn(acc[4 * j], v.x);
+            acc[4 * j + 1] = pc == 0 ? v.y : __fadd_rn(acc[4 * j + 1], v.y);
+            acc[4 * j + 2] = pc == 0 ? v.z : __fadd_rn(acc[4 * j + 2], v.z);
+            acc[4 * j + 3] = pc == 0 ? v.w : __fadd_rn(acc[4 * j + 3], v.w);
+          }
+        }
+        uint32_t r[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(acc[j]);
+        const int krow = tile0 * kTileM + (u & 3) * 32 + lane, kcol0 = (u >> 2) * 16;
+        if (krow < p.Mk) decode_store_chunk<16>(e, r, krow, kcol0, min(16, p.Nk - kcol0));
+      }
     }
   }
 
   DECODE_STAMP(p, 7, warp == 6 && lane == 0);
+  if (splits > 1 && *abort_flag != 0 && threadIdx.x == 0) {
+    // pieces that were on their way when this CTA gave up waiting for them: time to land
+    const uint64_t t_end = global_timer_ns() + 200000;
+    while (global_timer_ns() < t_end) __nanosleep(1000);
+  }
   tc_fence_before_sync();
+  __syncwarp();
+  if (splits > 1) {
+    // No CTA leaves while another may still send to it (which the waits above imply, unless one
+    // of them gave up).
+    if (warp < 6) {
+      cluster_wait();
+      cluster_arrive();
+    }
+    cluster_wait();
+  }
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, static_cast<uint32_t>(p.tmem_cols));
 }

@@ -151,7 +151,7 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, uint32_t (&r)[3
   }
 #pragma unroll
   for (int i = 0; i < 32; ++i) r[i] = linear_combine_bits<kInt>(e, r[i], src[i]);
-  for (int t = 0; t < e.n_ops; ++t) apply_op_chunk<kInt>(e.ops[t], r, krow, kcol0, ncols);
+  for (int t = 0; t < e.n_ops; ++t) apply_op_chunk<kInt, 32>(e.ops[t], r, krow, kcol0, ncols);
   if (d_smem_row != 0) {
     // same 16-byte-piece swizzle as the TMA box (row & 7)
 #pragma unroll

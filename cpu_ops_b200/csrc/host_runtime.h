@@ -77,8 +77,6 @@ struct TensorMapSlot {
 };
 constexpr int kTensorMapSlots = 64;
 
-constexpr int kDecodeMaxTiles = 4096;  // 128-row weight tiles the decode kernel's counters cover
-
 struct DeviceState {
   std::mutex mu;                  // held across a call's launches and its synchronisation
   std::atomic<bool> ready{false};
@@ -104,7 +102,6 @@ struct DeviceState {
     void* ptr = nullptr;
     size_t bytes = 0;
     bool captured = false;
-    int32_t* counters = nullptr;  // decode kernel: arrival counters, zero between launches
   };
   std::map<cudaStream_t, Workspace> ws;
   std::vector<void*> retired;
@@ -117,6 +114,8 @@ struct DeviceState {
   // Largest number of two-CTA clusters of the pair kernel that can be resident at once,
   // per kind (-1: not asked yet; 0: cluster launch unavailable).
   int pair_clusters[3] = {-1, -1, -1};
+  // The same for the decode kernel's clusters, by cluster size.
+  int decode_clusters[kDecodeMaxSplits + 1] = {-1, -1, -1, -1, -1, -1, -1};
   TensorMapSlot tm_cache[kTensorMapSlots];
 };
 
@@ -315,29 +314,6 @@ int ensure_workspace(DeviceState& st, cudaStream_t stream, size_t bytes, uint8_t
   return 0;
 }
 
-// The stream's arrival counters for the decode kernel (zero whenever no launch is in flight).
-int ensure_counters(DeviceState& st, cudaStream_t stream, int32_t** out) {
-  DeviceState::Workspace& w = st.ws[stream];
-  if (!w.counters) {
-    if (stream_is_capturing(stream)) {
-      set_error("the first small-m MX call on a stream must run outside stream capture (it allocates "
-                "its arrival counters)");
-      return CPUOPS_B200_STATUS_INVALID_ARGUMENTS;
-    }
-    CUDA_TRY(cudaMalloc(&w.counters, kDecodeMaxTiles * 4 * sizeof(int32_t)));
-    CUDA_TRY(cudaMemsetAsync(w.counters, 0, kDecodeMaxTiles * 4 * sizeof(int32_t), stream));
-  }
-  *out = w.counters;
-  return 0;
-}
-
-// After a device-side timeout the counters of an interrupted launch may be left non-zero.
-void reset_counters(DeviceState& st, cudaStream_t stream) {
-  auto it = st.ws.find(stream);
-  if (it != st.ws.end() && it->second.counters)
-    cudaMemsetAsync(it->second.counters, 0, kDecodeMaxTiles * 4 * sizeof(int32_t), stream);
-}
-
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Launch-policy overrides for A/B measurements.  They exist only in a library built with
@@ -357,15 +333,14 @@ struct EnvSwitches {
   int epi_warps = geti("CPUOPS_B200_EPI_WARPS", 0);
   bool no_decode = getenv("CPUOPS_B200_NO_DECODE") != nullptr;
   bool no_pdl = getenv("CPUOPS_B200_NO_PDL") != nullptr;
-  int decode_grid = geti("CPUOPS_B200_DECODE_GRID", 0);
+  int decode_splits = geti("CPUOPS_B200_DECODE_SPLITS", 0);
   int decode_stages = geti("CPUOPS_B200_DECODE_STAGES", 0);
-  int decode_ctas_per_sm = geti("CPUOPS_B200_DECODE_CTAS_PER_SM", 0);
   int producers = geti("CPUOPS_B200_PRODUCERS", 0);
 #else
   static constexpr bool no_c_ring = false, no_d_tma = false, clk = false, no_narrow = false,
                         no_decode = false, no_pdl = false;
-  static constexpr int panels = 0, raster_m = 0, pair = -1, ring = 0, epi_warps = 0, decode_grid = 0,
-                       decode_stages = 0, decode_ctas_per_sm = 0, producers = 0;
+  static constexpr int panels = 0, raster_m = 0, pair = -1, ring = 0, epi_warps = 0, decode_splits = 0,
+                       decode_stages = 0, producers = 0;
 #endif
 };
 const EnvSwitches& env_switches() {

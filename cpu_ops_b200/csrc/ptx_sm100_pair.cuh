@@ -23,6 +23,15 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The two halves of cluster_sync_all, for work in between.  Every thread of the cluster takes
+// both, in turn.
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void fence_mbar_init_cluster() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -38,6 +47,16 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 // Arrive on a barrier that may live in the other CTA (`bar` from map_to_cta).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// 16 bytes into shared memory of a CTA of the cluster (`dst`, `bar` from map_to_cta, both in
+// the same CTA); the bytes are credited to `bar` when they have been written.
+__device__ __forceinline__ void st_async_v4(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d,
+                                            uint32_t bar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+      "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar)
+      : "memory");
 }
 
 // Tiled TMA load into this CTA's shared memory, issued by the lane with `issue` != 0 of

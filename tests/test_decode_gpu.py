@@ -83,6 +83,29 @@ def test_never_split_keeps_whole_tiles(gpu, oracle):
     assert np.array_equal(D0.view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("fmt", [FMT_E2M1, FMT_E4M3])
+@pytest.mark.parametrize("m", [1, 17, 64])
+@pytest.mark.parametrize("n,kb,slices", [(128, 3, 1), (130, 20, 6), (1000, 9, 3), (1000, 19, 6), (2600, 23, 6),
+                                         (3584, 16, 4), (7160, 25, 2), (7160, 23, 1)])
+def test_k_cut_over_a_cluster(gpu, oracle, fmt, m, n, kb, slices):
+    """Every cluster size, k-blocks that do not divide by it, a ragged last k-block, and from
+    one to sixteen (lane quarter x 16 column) units for the CTAs of the cluster to own."""
+    per = 256 if fmt == FMT_E2M1 else 128
+    k = kb * per - 32
+    P = W.mx_problem(fmt, m, n, k, True, lds=lds16(k), scale_lo=118, scale_hi=122, seed=0xC0 + m + n + kb)
+    bias = W.rng_for(4, 3).standard_normal(n).astype(np.float32)
+    st, D = run_mx_gpu(P, 1.0, 0.5, chain=[c.BiasAdd(bias)])
+    assert st == c.Status.kSuccess, _capi.last_error()
+    plan = _capi.last_plan()
+    assert plan.decode == 1 and plan.slices == slices, plan.slices
+    want = run_mx_oracle(oracle, P, 1.0, 0.5, ops=[(OP_BIAS_ADD, bias, 0.0, 0.0)])
+    G, R = gather(D, m, n, P.ldc, True), gather(want, m, n, P.ldc, True)
+    assert not np.isnan(G).any()
+    assert normwise(G, R) <= MX_TOL
+    st, D2 = run_mx_gpu(P, 1.0, 0.5, chain=[c.BiasAdd(bias)])
+    assert np.array_equal(D.view(np.uint32), D2.view(np.uint32)), "run-to-run bits differ"
+
+
 def test_scale_arrays_tma_cannot_address_take_the_general_kernel(gpu, oracle):
     """A scale leading dimension that is not a multiple of 16 is legal (mx_formats.h:280-295
     only asks ld_scales >= ceil(k/32)); the call then runs the general kernel."""
