@@ -404,6 +404,25 @@ static int launch_relayout(const void* src0, void* dst0, const ScaleLayout& L0, 
   return 0;
 }
 
+// Copies one or two operands into aligned rows (j1.rows == 0: one).
+static int launch_repack(const RepackJob& j0, const RepackJob& j1, cudaStream_t stream) {
+  const int64_t items = repack_work_items(j0) + (j1.rows > 0 ? repack_work_items(j1) : 0);
+  const int threads = 256;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(std::min<int64_t>((items * 32 + threads - 1) / threads, 148 * 8)));
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = env_switches().no_pdl ? 0 : 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, repack_rows_kernel, j0, j1));
+  g_launches.fetch_add(1);
+  CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
 CPUOPS_B200_API int cpuops_b200_relayout_scales(const void* scales, int32_t rows, int32_t k,
                                                 int32_t ld_scales, int32_t tile_rows,
                                                 int32_t blocks_per_stage, void* out, void* stream) {
@@ -906,45 +925,31 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   const uint8_t* c_ptr = static_cast<const uint8_t*>(d->c);
   uint8_t* d_ptr = static_cast<uint8_t*>(d->d);
   if (k > 0) {
+    RepackJob jobs[2] = {};
+    int n_jobs = 0;
+    const int a_rows = static_cast<int>(A.outer), a_row_bytes = static_cast<int>(A.inner_bytes);
+    const int b_rows = static_cast<int>(B.outer), b_row_bytes = static_cast<int>(B.inner_bytes);
     if (!a_dev) {
       CUDA_TRY(cudaMemcpy2DAsync(wsp + off_a, a_pitch_dev, d->a, A.pitch, A.inner_bytes, A.outer,
                                  cudaMemcpyHostToDevice, stream));
       a_ptr = wsp + off_a;
-      if (a_mask) {  // clear the out-of-range nibble of an odd-k fp4 row in place
-        repack_rows_kernel<<<std::min<int64_t>((A.outer * ((A.inner_bytes + 15) / 16) + 255) / 256, 2368),
-                             256, 0, stream>>>(a_ptr, a_pitch_dev, wsp + off_a, a_pitch_dev,
-                                               static_cast<int>(A.outer),
-                                               static_cast<int>(A.inner_bytes), 1);
-        g_launches.fetch_add(1);
-      }
+      // (an odd-k fp4 row's out-of-range nibble is cleared in place)
+      if (a_mask) jobs[n_jobs++] = RepackJob{a_ptr, wsp + off_a, a_pitch_dev, a_pitch_dev, a_rows, a_row_bytes, 1};
     } else if (a_repack) {
-      repack_rows_kernel<<<static_cast<unsigned>(std::min<int64_t>(
-                               (A.outer * ((A.inner_bytes + 15) / 16) + 255) / 256, 2368)),
-                           256, 0, stream>>>(a_ptr, A.pitch, wsp + off_a, a_pitch_dev,
-                                             static_cast<int>(A.outer),
-                                             static_cast<int>(A.inner_bytes), a_mask ? 1 : 0);
-      g_launches.fetch_add(1);
+      jobs[n_jobs++] = RepackJob{a_ptr, wsp + off_a, A.pitch, a_pitch_dev, a_rows, a_row_bytes, a_mask ? 1 : 0};
       a_ptr = wsp + off_a;
     }
     if (!b_dev) {
       CUDA_TRY(cudaMemcpy2DAsync(wsp + off_b, b_pitch_dev, d->b, B.pitch, B.inner_bytes, B.outer,
                                  cudaMemcpyHostToDevice, stream));
       b_ptr = wsp + off_b;
-      if (b_mask) {
-        repack_rows_kernel<<<std::min<int64_t>((B.outer * ((B.inner_bytes + 15) / 16) + 255) / 256, 2368),
-                             256, 0, stream>>>(b_ptr, b_pitch_dev, wsp + off_b, b_pitch_dev,
-                                               static_cast<int>(B.outer),
-                                               static_cast<int>(B.inner_bytes), 1);
-        g_launches.fetch_add(1);
-      }
+      if (b_mask) jobs[n_jobs++] = RepackJob{b_ptr, wsp + off_b, b_pitch_dev, b_pitch_dev, b_rows, b_row_bytes, 1};
     } else if (b_repack) {
-      repack_rows_kernel<<<static_cast<unsigned>(std::min<int64_t>(
-                               (B.outer * ((B.inner_bytes + 15) / 16) + 255) / 256, 2368)),
-                           256, 0, stream>>>(b_ptr, B.pitch, wsp + off_b, b_pitch_dev,
-                                             static_cast<int>(B.outer),
-                                             static_cast<int>(B.inner_bytes), b_mask ? 1 : 0);
-      g_launches.fetch_add(1);
+      jobs[n_jobs++] = RepackJob{b_ptr, wsp + off_b, B.pitch, b_pitch_dev, b_rows, b_row_bytes, b_mask ? 1 : 0};
       b_ptr = wsp + off_b;
+    }
+    if (n_jobs > 0) {
+      if (int rc = launch_repack(jobs[0], jobs[1], stream)) return rc;
     }
     if (is_mx && !sa_dev) {
       CUDA_TRY(cudaMemcpyAsync(wsp + off_sa, d->a_scales, static_cast<size_t>(m - 1) * d->ld_scales_a + (k + 31) / 32,
@@ -1268,22 +1273,32 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
         return CPUOPS_B200_STATUS_CUDA_ERROR;
       }
     }
-    // C through a TMA-fed shared-memory ring when it is row-contiguous in kernel view and
-    // addressable by TMA; otherwise the epilogue loads it directly.
+    // C and D through the epilogue's shared-memory ring: by TMA where it can address them,
+    // else in rows (or columns) of 32 words; a D whose rows are the contiguous direction in
+    // kernel view is stored straight from the accumulator's lanes, which hold a row each.
     CUtensorMap tmC = tmA;
-    if (p.mode == kModeEpilogue && beta_nonzero && epi.c_sc == 1 &&
-        tma_addressable(epi.C, epi.c_sr * 4, Mk) && !env_switches().no_c_ring) {
-      if (int rc = make_tensor_map_words(&tmC, epi.C, Nk, Mk, epi.c_sr * 4)) return rc;
-      p.c_ring = 1;
+    if (p.mode == kModeEpilogue && beta_nonzero && !env_switches().no_c_ring) {
+      if (epi.c_sc != 1) {
+        if (epi.c_sr == 1) p.c_ring = kRingColumns;
+      } else if (tma_addressable(epi.C, epi.c_sr * 4, Mk)) {
+        if (int rc = make_tensor_map_words(&tmC, epi.C, Nk, Mk, epi.c_sr * 4)) return rc;
+        p.c_ring = kRingTma;
+      } else {
+        p.c_ring = kRingRows;
+      }
     }
-    // D through the same ring by TMA store when it is row-contiguous and addressable.
     CUtensorMap tmD = tmA;
-    if (p.mode == kModeEpilogue && epi.d_sc == 1 && tma_addressable(epi.D, epi.d_sr * 4, Mk) &&
-        !env_switches().no_d_tma) {
-      if (int rc = make_tensor_map_words(&tmD, epi.D, Nk, Mk, epi.d_sr * 4)) return rc;
-      p.d_tma = 1;
+    if (p.mode == kModeEpilogue && epi.d_sc == 1 && !env_switches().no_d_tma) {
+      // (a TMA store writes whole 16-byte pieces: up to three words behind the last column of a
+      // row whose length is not a multiple of four, which only the library's own buffer may take)
+      if (tma_addressable(epi.D, epi.d_sr * 4, Mk) && (Nk % 4 == 0 || !d_dev)) {
+        if (int rc = make_tensor_map_words(&tmD, epi.D, Nk, Mk, epi.d_sr * 4)) return rc;
+        p.d_ring = kRingTma;
+      } else {
+        p.d_ring = kRingRows;
+      }
     }
-    p.ring_bufs = (p.c_ring || p.d_tma) ? 2 : 0;
+    p.ring_bufs = (p.c_ring || p.d_ring) ? 2 : 0;
     if (p.ring_bufs && env_switches().ring == 3) p.ring_bufs = 3;
     // Eight epilogue warps (two per tensor-memory lane quarter) when no CTA gets a second
     // tile to hide its epilogue behind and the tile is wide enough to share out; otherwise
@@ -1405,7 +1420,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     g_last_plan.slices = ch.slices;
     g_last_plan.stages = stages;
     g_last_plan.grid = static_cast<int32_t>(grid);
-    g_last_plan.c_ring = p.c_ring;
+    g_last_plan.c_ring = p.c_ring == kRingTma ? 1 : 0;
     g_last_plan.prepared_b = used_prepared ? 1 : 0;
     g_last_plan.epilogue_warps = epi_warps;
     g_last_plan.narrow_last = p.narrow_last;

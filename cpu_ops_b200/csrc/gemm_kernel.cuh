@@ -101,9 +101,67 @@ __device__ __forceinline__ bool aligned16(const void* ptr) {
   return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0;
 }
 
+// One word of C, global -> shared, without a register in between (zero when not `valid`;
+// nothing is read then).  `src` is a 4-byte aligned address.
+__device__ __forceinline__ void copy_word_async(uint32_t dst, const uint32_t* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+
+// Byte offset of word `col` of row `row` in a ring buffer (rows of 128 bytes, 16-byte pieces
+// XOR-swizzled by row & 7, as TMA lays a 128-byte swizzled box out).
+__device__ __forceinline__ uint32_t ring_word(int row, int col) {
+  return static_cast<uint32_t>(row * 128 + (((col >> 2) ^ (row & 7)) << 4) + (col & 3) * 4);
+}
+
+// Fetches a 32 x 32 chunk of C that TMA cannot address (its base or leading dimension is not a
+// multiple of 16 bytes, or its columns are the contiguous direction) into a ring buffer; the
+// caller commits the group.  By rows: one 128-byte row per instruction, laid out as TMA
+// would.  By columns (kRingColumns): lane = row, every lane fetches the words that it will use.
+__device__ __forceinline__ void fetch_c_chunk(const GemmParams& p, uint32_t buf, int row0, int kcol0, int lane) {
+  const EpilogueParams& e = p.epi;
+  const uint32_t* base = static_cast<const uint32_t*>(e.C) + (row0 * e.c_sr + kcol0 * e.c_sc);
+  const int nrows = p.Mk - row0, ncols = p.Nk - kcol0;  // what the matrix still has from here on
+  if (p.c_ring == kRingRows) {
+    const uint32_t* src = base + (lane < ncols ? lane : 0);
+#pragma unroll
+    for (int r = 0; r < 32; ++r, src += e.c_sr) {
+      const bool valid = r < nrows && lane < ncols;
+      copy_word_async(buf + ring_word(r, lane), valid ? src : static_cast<const uint32_t*>(e.C), valid);
+    }
+  } else {
+    const uint32_t* src = base + lane;
+#pragma unroll
+    for (int i = 0; i < 32; ++i, src += e.c_sc) {
+      const bool valid = lane < nrows && i < ncols;
+      copy_word_async(buf + static_cast<uint32_t>(i * 128 + lane * 4),
+                      valid ? src : static_cast<const uint32_t*>(e.C), valid);
+    }
+  }
+}
+
+// Writes a finished chunk from a ring buffer to a D that TMA cannot address: one row of up to
+// 32 words per instruction.  (From the accumulator's lanes, which hold a row each, every store
+// instruction would touch 32 lines, four bytes of each.)
+__device__ __forceinline__ void write_d_rows(const GemmParams& p, uint32_t buf, int row0, int kcol0, int lane) {
+  const EpilogueParams& e = p.epi;
+  uint32_t* dst = static_cast<uint32_t*>(e.D) + (row0 * e.d_sr + kcol0 + lane);
+  const int nrows = lane < p.Nk - kcol0 ? p.Mk - row0 : 0;
+#pragma unroll
+  for (int r0 = 0; r0 < 32; r0 += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[j]) : "r"(buf + ring_word(r0 + j, lane)));
+#pragma unroll
+    for (int j = 0; j < 8; ++j, dst += e.d_sr)
+      if (r0 + j < nrows) *dst = v[j];
+  }
+}
+
 // Stores one 32-column chunk of one accumulator row.
 // `c_smem_row`: shared-memory address of this thread's row of the C chunk prefetched into
-// the ring, or 0.  `d_smem_row`: where to put the finished row for the TMA store, or 0
+// the ring, or 0 (kRingColumns: of the thread's first word, the next ones 128 bytes apart).
+// `d_smem_row`: where to put the finished row for the TMA store or write_d_rows, or 0
 // (store directly).  Explicit shared-space accesses: generic ones cost more.
 template <bool kInt>
 __device__ __forceinline__ void store_chunk(const GemmParams& p, uint32_t (&r)[32], int krow,
@@ -125,8 +183,12 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, uint32_t (&r)[3
   }
   const EpilogueParams& e = p.epi;
   uint32_t src[32];
-  if (c_smem_row != 0) {
-    // C chunk prefetched by TMA: this thread's row, 16-byte pieces XOR-swizzled by row & 7
+  if (c_smem_row != 0 && p.c_ring == kRingColumns) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(src[i]) : "r"(c_smem_row + 128u * i));
+  } else if (c_smem_row != 0) {
+    // C chunk prefetched by TMA or by rows: this thread's row, 16-byte pieces XOR-swizzled by row & 7
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
@@ -261,8 +323,8 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
   if (warp == 0 && lane == 0) {
     prefetch_tensormap(&tmA);
     prefetch_tensormap(&tmB);
-    if (p.c_ring) prefetch_tensormap(&tmC);
-    if (p.d_tma) prefetch_tensormap(&tmD);
+    if (p.c_ring == kRingTma) prefetch_tensormap(&tmC);
+    if (p.d_ring == kRingTma) prefetch_tensormap(&tmD);
     if constexpr (kMx && kPair) {
       prefetch_tensormap(&tmSFA);
       prefetch_tensormap(&tmSFB);
@@ -575,12 +637,16 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
     const int cstep = n_epi >> 2, c0 = ew >> 2;
     int it = 0;
     // Ring of two 4 KB chunk buffers per warp (32 rows x 32 words, 128-byte swizzled);
-    // chunk x uses buffer x % 2.  With c_ring, C chunks are fetched into it by TMA two
-    // chunks ahead of their use; with d_tma, the finished chunk is written into its
-    // buffer (in place over C) and leaves by TMA store, so D is written in whole 128-byte
+    // chunk x uses buffer x % 2.  With c_ring, C chunks are fetched into it two chunks
+    // ahead of their use; with d_ring, the finished chunk is written into its buffer (in
+    // place over C) and leaves by TMA store or row by row, so D is written in whole 128-byte
     // row pieces; a buffer is refilled only after the store that read it is done with it.
     // A third buffer (p.ring_bufs == 3) hides that wait at the price of shared memory.
-    const bool ring = p.c_ring != 0, d_tma = p.d_tma != 0;
+    // TMA carries what it can address; the rest goes through cp.async and plain stores
+    // (fetch_c_chunk, write_d_rows): 1999 x 3001 x 1777 with leading dimensions of dim + 3
+    // and beta = 1, 36.8 -> 29.3 us (with the copy of A and B below).
+    const bool ring = p.c_ring != kRingNone, d_tma = p.d_ring == kRingTma, d_rows = p.d_ring == kRingRows;
+    const bool c_tma = p.c_ring == kRingTma;
     const uint32_t nb = static_cast<uint32_t>(p.ring_bufs);
     asm volatile("griddepcontrol.wait;" ::: "memory");  // before C is read, D or a slab written
     warm_epilogue_params(p.epi);  // constant-cache misses now, not after the first accumulator
@@ -595,9 +661,13 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
     const long long edbg_start = edbg ? clock64() : 0;
     // pair: the leader's MMA thread waits for the epilogue warps of both CTAs
     const uint32_t acc_empty0 = kPair ? map_to_cta(acc_empty_bar(0), 0) : acc_empty_bar(0);
-    auto request_c = [&](int col, int row) {  // lane 0 only
-      mbar_expect_tx(c_full_bar(ew, ci_b), 4096u);
-      tma_load_2d(my_c + ci_b * 4096u, &tmC, c_full_bar(ew, ci_b), col, row);
+    auto request_c = [&](int col, int row) {  // TMA: lane 0 only; otherwise the whole warp
+      if (c_tma) {
+        mbar_expect_tx(c_full_bar(ew, ci_b), 4096u);
+        tma_load_2d(my_c + ci_b * 4096u, &tmC, c_full_bar(ew, ci_b), col, row);
+      } else {
+        fetch_c_chunk(p, my_c + ci_b * 4096u, row, col, lane);
+      }
       ++cissued;
       if (++ci_b == nb) ci_b = 0;
     };
@@ -609,10 +679,15 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
       const int krow = row0 + lane;
       const int n0 = tc.n_tile * p.BN;
       const int nchunks = tc.bn / 32;
-      if (ring && lane == 0) {
+      if (ring && (lane == 0 || !c_tma)) {
         // this warp's first two chunks of the tile: requested before the accumulator is ready
-        if (d_tma) bulk_wait_group_read<0>();
-        for (int c = c0; c < c0 + 2 * cstep && c < nchunks; c += cstep) request_c(n0 + c * 32, row0);
+        // (cp.async: always two groups, so that the count stays in step)
+        if (d_tma && lane == 0) bulk_wait_group_read<0>();
+        if (!c_tma) __syncwarp();
+        for (int c = c0; c < c0 + 2 * cstep; c += cstep) {
+          if (c < nchunks) request_c(n0 + c * 32, row0);
+          if (!c_tma) cp_async_commit();
+        }
       }
       const long long te0 = edbg ? clock64() : 0;
       const bool ready = mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
@@ -654,7 +729,11 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
         }
         const int kcol0 = n0 + c * 32;
         uint32_t c_row = 0, d_row = 0;  // shared-memory addresses of this lane's row
-        if (ring) {
+        if (ring && !c_tma) {
+          cp_async_wait<1>();  // all groups but the youngest: this chunk's
+          __syncwarp();        // ... of every lane
+          c_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * (p.c_ring == kRingColumns ? 4u : 128u);
+        } else if (ring) {
           const bool got = mbar_wait_bounded(c_full_bar(ew, cq_b), cq_ph, abort_flag, budget_ns);
           if (!__all_sync(0xffffffffu, got)) {
             if (lane == 0) record_error(p, abort_flag, kErrEpilogueWait);
@@ -669,7 +748,7 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
           }
           __syncwarp();
         }
-        if (d_tma) d_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * 128u;
+        if (d_tma || d_rows) d_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * 128u;
         if (krow < p.Mk && kcol0 < p.Nk)
           store_chunk<kInt>(p, r, krow, kcol0, tc.slice, c_row, d_row, lane & 7);
         if (d_tma) {
@@ -679,10 +758,14 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
             if (row0 < p.Mk && kcol0 < p.Nk) tma_store_2d(&tmD, my_c + cq_b * 4096u, kcol0, row0);
             bulk_commit_group();
           }
+        } else if (d_rows) {
+          __syncwarp();  // every lane's row is there
+          write_d_rows(p, my_c + cq_b * 4096u, row0, kcol0, lane);
+          __syncwarp();  // every lane has read its words: the buffer may be written again
         } else if (ring) {
           __syncwarp();  // every lane has read its row: the buffer may be refilled
         }
-        if (ring && lane == 0 && c + 2 * cstep < nchunks) {
+        if (ring && c_tma && lane == 0 && c + 2 * cstep < nchunks) {
           // chunk c + 2 goes where chunk c (two buffers) or chunk c - 1 (three) was: the
           // store out of that buffer must have read it first.  With three buffers that is
           // the store before the one just issued, which has normally finished by now.
@@ -690,6 +773,17 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
             if (nb >= 3) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
           }
           request_c(n0 + (c + 2 * cstep) * 32, row0);
+        } else if (ring && !c_tma) {
+          if (c + 2 * cstep < nchunks) {
+            if (d_tma) {  // (as above; lane 0 holds the bulk groups)
+              if (lane == 0) {
+                if (nb >= 3) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
+              }
+              __syncwarp();
+            }
+            request_c(n0 + (c + 2 * cstep) * 32, row0);
+          }
+          cp_async_commit();
         }
         ++cq;
         if (++cq_b == nb) {
@@ -703,7 +797,8 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
       B200_CLK(p)[5] = static_cast<unsigned long long>(clock64() - edbg_start);
       B200_CLK(p)[6] = static_cast<unsigned long long>(edbg_wait);
     }
-    if (ring && *abort_flag != 0 && lane == 0) {
+    if (ring && !c_tma) cp_async_wait<0>();
+    if (c_tma && *abort_flag != 0 && lane == 0) {
       // let C chunks that were requested but never consumed land before the CTA exits
       int dummy = 0;
       for (; cq < cissued; ++cq) {

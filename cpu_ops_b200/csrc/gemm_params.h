@@ -19,6 +19,11 @@ constexpr int kMaxStages = 8;
 
 enum : int32_t { kKindI8 = 0, kKindMxf8 = 1, kKindMxf4 = 2 };
 enum : int32_t { kModeEpilogue = 0, kModePartial = 1 };
+// How chunks of C reach the epilogue's shared-memory ring, and how finished chunks of D leave
+// it: not at all (plain loads and stores by the accumulator's lanes), by TMA, by 128-byte rows
+// (cp.async / plain stores, for bases and leading dimensions that TMA cannot address), or - C
+// only - by columns (lane = row, where the rows are the contiguous direction).
+enum : int32_t { kRingNone = 0, kRingTma = 1, kRingRows = 2, kRingColumns = 3 };
 enum : int32_t {
   kOpRelu = 1, kOpClamp = 2, kOpBiasAdd = 3, kOpScalePerRow = 4, kOpScalePerCol = 5,
   kOpGelu = 6, kOpSilu = 7
@@ -75,8 +80,8 @@ struct GemmParams {
   const uint8_t* sfa;
   const uint8_t* sfb;
   int32_t sfa_stage_bytes, sfb_stage_bytes;  // per k-block
-  int32_t c_ring;           // 1: C tiles are prefetched by TMA into a shared-memory ring
-  int32_t d_tma;            // 1: D chunks leave through that ring by TMA store
+  int32_t c_ring;           // kRing*: how C chunks are prefetched into a shared-memory ring
+  int32_t d_ring;           // kRing*: how D chunks leave through that ring
   int32_t ring_bufs;        // ring buffers per epilogue warp: 0 (no ring) or 2
   int32_t tx_operand_bytes; // bytes the A and B loads of one stage credit to the barrier, per CTA
   int32_t* error;           // device error word

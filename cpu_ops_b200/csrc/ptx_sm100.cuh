@@ -141,6 +141,12 @@ __device__ __forceinline__ void bulk_wait_group_read() {
 __device__ __forceinline__ void bulk_wait_group_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
+// cp.async (per-thread copies): close this thread's group; wait until at most N are pending.
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 // Generic-proxy writes to shared memory -> visible to the async proxy (TMA store source).
 __device__ __forceinline__ void fence_proxy_async_shared_cta() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
