@@ -404,6 +404,31 @@ static int launch_relayout(const void* src0, void* dst0, const ScaleLayout& L0, 
   return 0;
 }
 
+// D = epilogue(the slabs' sum, C); no slabs: k == 0.
+static int launch_reduce(bool is_mx, const EpilogueParams& epi, const uint32_t* ws, int slices, int64_t slab, int Mk,
+                         int Nk, int64_t ws_sr, int64_t ws_sc, int sms, cudaStream_t stream) {
+  const int threads = 256;
+  const int64_t total = static_cast<int64_t>(Mk) * Nk;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(
+      std::max<int64_t>(1, std::min<int64_t>((total + threads - 1) / threads, static_cast<int64_t>(sms) * 16))));
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = env_switches().no_pdl || g_profile.load() ? 0 : 1;
+  if (is_mx) {
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_epilogue_kernel<false>, epi, ws, slices, slab, Mk, Nk, ws_sr, ws_sc));
+  } else {
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_epilogue_kernel<true>, epi, ws, slices, slab, Mk, Nk, ws_sr, ws_sc));
+  }
+  g_launches.fetch_add(1);
+  CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
 // Copies one or two operands into aligned rows (j1.rows == 0: one).
 static int launch_repack(const RepackJob& j0, const RepackJob& j1, cudaStream_t stream) {
   const int64_t items = repack_work_items(j0) + (j1.rows > 0 ? repack_work_items(j1) : 0);
@@ -1006,24 +1031,9 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     memcpy(&o.hi, &op.hi, 4);
   }
 
-  const int ew_threads = 256;
-  auto ew_blocks = [&](int64_t total) {
-    return static_cast<unsigned>(std::max<int64_t>(
-        1, std::min<int64_t>((total + ew_threads - 1) / ew_threads, static_cast<int64_t>(sms) * 16)));
-  };
-
   if (k == 0) {
     // D = epilogue(0, C): run_blocked.h:30-36.  Kernel view == caller view here.
-    const int64_t sr = c_rm ? 1 : 0;  // compact order follows D's contiguous direction
-    if (is_mx) {
-      reduce_epilogue_kernel<false><<<ew_blocks(static_cast<int64_t>(m) * n), ew_threads, 0, stream>>>(
-          epi, nullptr, 0, 0, m, n, sr ? n : 1, sr ? 1 : m);
-    } else {
-      reduce_epilogue_kernel<true><<<ew_blocks(static_cast<int64_t>(m) * n), ew_threads, 0, stream>>>(
-          epi, nullptr, 0, 0, m, n, sr ? n : 1, sr ? 1 : m);
-    }
-    g_launches.fetch_add(1);
-    CUDA_TRY(cudaGetLastError());
+    if (int rc = launch_reduce(is_mx, epi, nullptr, 0, 0, m, n, c_rm ? n : 1, c_rm ? 1 : m, sms, stream)) return rc;
   } else if (dp.use) {
     // ---- decode kernel: W = the caller's B on the MMA M side, X = the caller's A ---------------
     CUtensorMap tmW, tmX;
@@ -1453,16 +1463,9 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       g_profile_events.emplace_back(ev0, ev1);
     }
     if (ch.slices > 1) {
-      const int64_t total = static_cast<int64_t>(Mk) * Nk;
-      if (is_mx) {
-        reduce_epilogue_kernel<false><<<ew_blocks(total), ew_threads, 0, stream>>>(
-            epi, static_cast<const uint32_t*>(p.ws), ch.slices, p.ws_slab, Mk, Nk, p.ws_sr, p.ws_sc);
-      } else {
-        reduce_epilogue_kernel<true><<<ew_blocks(total), ew_threads, 0, stream>>>(
-            epi, static_cast<const uint32_t*>(p.ws), ch.slices, p.ws_slab, Mk, Nk, p.ws_sr, p.ws_sc);
-      }
-      g_launches.fetch_add(1);
-      CUDA_TRY(cudaGetLastError());
+      if (int rc = launch_reduce(is_mx, epi, static_cast<const uint32_t*>(p.ws), ch.slices, p.ws_slab, Mk, Nk, p.ws_sr,
+                                 p.ws_sc, sms, stream))
+        return rc;
     }
   }
 
@@ -1722,13 +1725,8 @@ CPUOPS_B200_API int cpuops_b200_gemm_i8_noalloc(const cpuops_b200_gemm_desc* d) 
                                                                             tmA, tmA /*unused: MX pair only*/, p);
   g_launches.fetch_add(1);
   CUDA_TRY(cudaGetLastError());
-  const int64_t total = static_cast<int64_t>(m) * n;
-  const unsigned blocks = static_cast<unsigned>(
-      std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, static_cast<int64_t>(nd->sm_count) * 16)));
-  reduce_epilogue_kernel<true><<<blocks, 256, 0, stream>>>(epi, slabs, slices, p.ws_slab, m, n, p.ws_sr,
-                                                          p.ws_sc);
-  g_launches.fetch_add(1);
-  CUDA_TRY(cudaGetLastError());
+  if (int rc = launch_reduce(false, epi, slabs, slices, p.ws_slab, m, n, p.ws_sr, p.ws_sc, nd->sm_count, stream))
+    return rc;
 
   int32_t device_error = 0;
   CUDA_TRY(cudaMemcpyAsync(&device_error, error_word, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));

@@ -138,32 +138,40 @@ __global__ void relayout_scales_kernel(const uint8_t* __restrict__ src0, uint8_t
 // ((w0 + w1) + w2) + ..., as the CPU library's reduce_splitk does
 // (gemm/kernel/run_blocked.h:40-75); slices == 0 is its write_zero_k (:30-36).
 // Threads walk the slab's compact order, which the launcher chooses to match
-// the contiguous direction of D.
+// the contiguous direction of D.  A thread's slab words are independent loads, eight of them in
+// flight: with one element per thread the kernel is bound by that latency, and by the gap
+// between two launches, which programmatic stream serialization hides (192 x 320 x 16384 u8 x s8 in 22 slices, both kernels: 14.35 -> 13.6 us).
 template <bool kInt>
-__global__ void reduce_epilogue_kernel(EpilogueParams e, const uint32_t* __restrict__ ws, int slices,
-                                       int64_t slab, int Mk, int Nk, int64_t ws_sr, int64_t ws_sc) {
+__global__ void __launch_bounds__(256) reduce_epilogue_kernel(EpilogueParams e, const uint32_t* ws, int slices,
+                                                              int64_t slab, int Mk, int Nk, int64_t ws_sr,
+                                                              int64_t ws_sc) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int64_t total = static_cast<int64_t>(Mk) * Nk;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const bool by_rows = ws_sc == 1;
+  const int line = by_rows ? Nk : Mk;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the slabs are written
   for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
        idx += stride) {
-    int krow, kcol;
-    if (ws_sc == 1) {
-      krow = static_cast<int>(idx / Nk);
-      kcol = static_cast<int>(idx - static_cast<int64_t>(krow) * Nk);
-    } else {
-      kcol = static_cast<int>(idx / Mk);
-      krow = static_cast<int>(idx - static_cast<int64_t>(kcol) * Mk);
-    }
+    const int outer = static_cast<int>(idx / line), inner = static_cast<int>(idx - static_cast<int64_t>(outer) * line);
+    const int krow = by_rows ? outer : inner, kcol = by_rows ? inner : outer;
     uint32_t acc = 0;
     if (slices > 0) {
       const uint32_t* w = ws + (krow * ws_sr + kcol * ws_sc);
-      acc = w[0];
-      for (int s = 1; s < slices; ++s) {
-        const uint32_t v = w[s * slab];
-        if constexpr (kInt) {
-          acc += v;
-        } else {
-          acc = __float_as_uint(__fadd_rn(__uint_as_float(acc), __uint_as_float(v)));
+      for (int s0 = 0; s0 < slices; s0 += 8) {
+        uint32_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = s0 + j < slices ? __ldcg(w + (s0 + j) * slab) : 0u;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (s0 + j >= slices) break;
+          if (s0 + j == 0) {
+            acc = v[0];
+          } else if constexpr (kInt) {
+            acc += v[j];
+          } else {
+            acc = __float_as_uint(__fadd_rn(__uint_as_float(acc), __uint_as_float(v[j])));
+          }
         }
       }
     }
