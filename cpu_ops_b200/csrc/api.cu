@@ -471,16 +471,7 @@ CPUOPS_B200_API int cpuops_b200_stream_status(void* stream) {
   if (int rc = init_device(-1, &st)) return rc;
   std::lock_guard<std::mutex> lk(st->mu);
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : st->stream;
-  CUDA_TRY(cudaMemcpyAsync(st->error_host, st->error_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaStreamSynchronize(s));
-  if (*st->error_host != 0) {
-    set_error("device-side bounded wait timed out (code %d)", *st->error_host);
-    *st->error_host = 0;
-    CUDA_TRY(cudaMemsetAsync(st->error_dev, 0, sizeof(int32_t), s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    return CPUOPS_B200_STATUS_DEVICE_TIMEOUT;
-  }
-  return 0;
+  return finish_stream(*st, s);
 }
 
 CPUOPS_B200_API int cpuops_b200_set_sm_limit(int32_t device, int32_t sms) {
@@ -509,16 +500,7 @@ CPUOPS_B200_API int cpuops_b200_selftest_wait_timeout(uint32_t budget_us, void* 
   wait_timeout_probe_kernel<<<1, 32, 0, s>>>(st->error_dev, budget_us);
   g_launches.fetch_add(1);
   CUDA_TRY(cudaGetLastError());
-  CUDA_TRY(cudaMemcpyAsync(st->error_host, st->error_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaStreamSynchronize(s));
-  if (*st->error_host != 0) {
-    set_error("device-side bounded wait timed out (code %d)", *st->error_host);
-    *st->error_host = 0;
-    CUDA_TRY(cudaMemsetAsync(st->error_dev, 0, sizeof(int32_t), s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    return CPUOPS_B200_STATUS_DEVICE_TIMEOUT;
-  }
-  return CPUOPS_B200_STATUS_SUCCESS;
+  return finish_stream(*st, s);
 }
 
 CPUOPS_B200_API int cpuops_b200_profile(int enable) {
@@ -636,16 +618,7 @@ static int run_host_row_panels(const cpuops_b200_gemm_desc* d, DeviceState& st, 
     CUDA_TRY(cudaEventRecord(st.panel_done[j], st.panel_stream[j]));
     CUDA_TRY(cudaStreamWaitEvent(stream, st.panel_done[j], 0));
   }
-  CUDA_TRY(cudaMemcpyAsync(st.error_host, st.error_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-  CUDA_TRY(cudaStreamSynchronize(stream));
-  if (*st.error_host != 0) {
-    set_error("device-side bounded wait timed out (code %d)", *st.error_host);
-    *st.error_host = 0;
-    cudaMemsetAsync(st.error_dev, 0, sizeof(int32_t), stream);
-    cudaStreamSynchronize(stream);
-    return CPUOPS_B200_STATUS_DEVICE_TIMEOUT;
-  }
-  return CPUOPS_B200_STATUS_SUCCESS;
+  return finish_stream(st, stream);
 }
 
 // Descriptor checks that need no device, in the CPU library's order (gemm.h:100-122,
@@ -1475,16 +1448,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   }
   if (async) return CPUOPS_B200_STATUS_SUCCESS;
 
-  CUDA_TRY(cudaMemcpyAsync(st.error_host, st.error_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-  CUDA_TRY(cudaStreamSynchronize(stream));
-  if (*st.error_host != 0) {
-    set_error("device-side bounded wait timed out (code %d)", *st.error_host);
-    *st.error_host = 0;
-    cudaMemsetAsync(st.error_dev, 0, sizeof(int32_t), stream);
-    cudaStreamSynchronize(stream);
-    return CPUOPS_B200_STATUS_DEVICE_TIMEOUT;
-  }
-  return CPUOPS_B200_STATUS_SUCCESS;
+  return finish_stream(st, stream);
 }
 
 // =================================================================================

@@ -27,7 +27,7 @@ __global__ void wait_timeout_probe_kernel(int32_t* error, uint32_t budget_us) {
   }
   __syncwarp();
   const bool done = mbar_wait_bounded(bar_addr, 0, &abort_flag, static_cast<uint64_t>(budget_us) * 1000ull);
-  if (!__all_sync(0xffffffffu, done) && threadIdx.x == 0) atomicCAS(error, 0, kErrProducerWait);
+  if (!__all_sync(0xffffffffu, done) && threadIdx.x == 0) leave_error(error, kErrProducerWait);
 }
 
 // Scale layout consumed by tcgen05.cp (32x128b.warpx4) + block-scaled MMAs.

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
     for (int i = 0; i < n_units; ++i) {
       if (!__all_sync(0xffffffffu, mbar_wait_bounded(empty_bar(s), ph ^ 1u, abort_flag, budget_ns))) {
         if (el) {
-          atomicCAS(p.error, 0, kErrProducerWait);
+          leave_error(p.error, kErrProducerWait);
           *abort_flag = 1;
         }
         break;
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       const int piece_units = kb1 - kb0;  // one tile
       if (!__all_sync(kAll, mbar_wait_bounded(acc_empty_bar(buf), acc_ph ^ 1u, abort_flag, budget_ns))) {
         if (el) {
-          atomicCAS(p.error, 0, kErrMmaWaitAcc);
+          leave_error(p.error, kErrMmaWaitAcc);
           *abort_flag = 1;
         }
         ok = false;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
         // the stage's operand tiles have landed and its scale atoms are written
         if (!__all_sync(kAll, mbar_wait_bounded(full_bar(s), ph, abort_flag, budget_ns))) {
           if (el) {
-            atomicCAS(p.error, 0, kErrMmaWaitFull);
+            leave_error(p.error, kErrMmaWaitFull);
             *abort_flag = 1;
           }
           ok = false;
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
     tc_commit_g<false>(drain_bar, el);
     int dummy = 0;
     if (!__all_sync(kAll, mbar_wait_bounded(drain_bar, 0, &dummy, budget_ns)) && el) {
-      atomicCAS(p.error, 0, kErrDrainWait);
+      leave_error(p.error, kErrDrainWait);
       *abort_flag = 1;
     }
     __syncwarp();
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
         // the stage's previous atoms have been copied to tensor memory (its MMAs are done)
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(empty_bar(s2), ph2 ^ 1u, abort_flag, budget_ns))) {
           if (lane == 0) {
-            atomicCAS(p.error, 0, kErrProducerWait);
+            leave_error(p.error, kErrProducerWait);
             *abort_flag = 1;
           }
           alive = false;
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       const bool got = mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
       if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) {
-          atomicCAS(p.error, 0, kErrEpilogueWait);
+          leave_error(p.error, kErrEpilogueWait);
           *abort_flag = 1;
         }
         alive = false;
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
         const bool got = mbar_wait_bounded(red_bar(slot), 0, abort_flag, budget_ns);
         if (!__all_sync(0xffffffffu, got)) {
           if (lane == 0) {
-            atomicCAS(p.error, 0, kErrEpilogueWait);
+            leave_error(p.error, kErrEpilogueWait);
             *abort_flag = 1;
           }
           break;

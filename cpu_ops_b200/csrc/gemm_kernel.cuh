@@ -92,7 +92,7 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int t, int
 
 __device__ __forceinline__ void record_error(const GemmParams& p, volatile int* abort_flag,
                                              int code) {
-  atomicCAS(p.error, 0, code);
+  leave_error(p.error, code);
   *abort_flag = 1;
   __threadfence_block();
 }

@@ -102,6 +102,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   return true;
 }
 
+// Leaves `code` in the call's error word unless one is there.  The word may be host memory
+// (no atomics over the bus: of two codes at the same moment either may stay).
+__device__ __forceinline__ void leave_error(int32_t* word, int32_t code) {
+  volatile int32_t* w = word;
+  if (*w == 0) *w = code;
+  __threadfence_system();
+}
+
 // ---- TMA ----------------------------------------------------------------------
 
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* tm) {
