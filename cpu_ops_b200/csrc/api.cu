@@ -567,15 +567,12 @@ static int run_host_row_panels(const cpuops_b200_gemm_desc* d, DeviceState& st, 
   }
   cpuops_b200_gemm_desc sub = *d;
   if (!b_dev) {
-    CUDA_TRY(cudaMemcpy2DAsync(bw + pb, b_pitch_staged, d->b, B.pitch, B.inner_bytes, B.outer,
-                               cudaMemcpyHostToDevice, stream));
+    if (int rc = upload_rows(st, stream, bw + pb, b_pitch_staged, d->b, B.pitch, B.inner_bytes, B.outer)) return rc;
     sub.b = bw + pb;
     sub.ldb = static_cast<int32_t>(fp4_b ? b_pitch_staged * 2 : b_pitch_staged);
   }
   if (is_mx && !sb_dev) {
-    CUDA_TRY(cudaMemcpyAsync(bw + psb, d->b_scales,
-                             static_cast<size_t>(n - 1) * d->ld_scales_b + (k + 31) / 32,
-                             cudaMemcpyHostToDevice, stream));
+    if (int rc = upload_rows(st, stream, bw + psb, static_cast<size_t>(n - 1) * d->ld_scales_b + (k + 31) / 32, d->b_scales, static_cast<size_t>(n - 1) * d->ld_scales_b + (k + 31) / 32, static_cast<size_t>(n - 1) * d->ld_scales_b + (k + 31) / 32, 1)) return rc;
     sub.b_scales = bw + psb;
   }
   CUDA_TRY(cudaEventRecord(st.fork_event, stream));
@@ -717,6 +714,13 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     device_lock = std::unique_lock<std::mutex>(st.mu);
     t_tm_cache = st.tm_cache;
   }
+  // (a call that returns early leaves no download behind that would write to its caller's memory later)
+  struct ForgetDownloads {
+    StagingRing* ring;
+    ~ForgetDownloads() {
+      if (ring) ring->forget();
+    }
+  } forget_downloads{depth == 0 ? &st.staging : nullptr};
   cudaStream_t stream = d->stream ? static_cast<cudaStream_t>(d->stream) : st.stream;
   const bool async = (d->flags & CPUOPS_B200_FLAG_ASYNC) != 0;
   const int sms = st.sms();  // SMs this call may occupy (cpuops_b200_set_sm_limit)
@@ -928,8 +932,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     const int a_rows = static_cast<int>(A.outer), a_row_bytes = static_cast<int>(A.inner_bytes);
     const int b_rows = static_cast<int>(B.outer), b_row_bytes = static_cast<int>(B.inner_bytes);
     if (!a_dev) {
-      CUDA_TRY(cudaMemcpy2DAsync(wsp + off_a, a_pitch_dev, d->a, A.pitch, A.inner_bytes, A.outer,
-                                 cudaMemcpyHostToDevice, stream));
+      if (int rc = upload_rows(st, stream, wsp + off_a, a_pitch_dev, d->a, A.pitch, A.inner_bytes, A.outer)) return rc;
       a_ptr = wsp + off_a;
       // (an odd-k fp4 row's out-of-range nibble is cleared in place)
       if (a_mask) jobs[n_jobs++] = RepackJob{a_ptr, wsp + off_a, a_pitch_dev, a_pitch_dev, a_rows, a_row_bytes, 1};
@@ -938,8 +941,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       a_ptr = wsp + off_a;
     }
     if (!b_dev) {
-      CUDA_TRY(cudaMemcpy2DAsync(wsp + off_b, b_pitch_dev, d->b, B.pitch, B.inner_bytes, B.outer,
-                                 cudaMemcpyHostToDevice, stream));
+      if (int rc = upload_rows(st, stream, wsp + off_b, b_pitch_dev, d->b, B.pitch, B.inner_bytes, B.outer)) return rc;
       b_ptr = wsp + off_b;
       if (b_mask) jobs[n_jobs++] = RepackJob{b_ptr, wsp + off_b, b_pitch_dev, b_pitch_dev, b_rows, b_row_bytes, 1};
     } else if (b_repack) {
@@ -950,19 +952,16 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       if (int rc = launch_repack(jobs[0], jobs[1], stream)) return rc;
     }
     if (is_mx && !sa_dev) {
-      CUDA_TRY(cudaMemcpyAsync(wsp + off_sa, d->a_scales, static_cast<size_t>(m - 1) * d->ld_scales_a + (k + 31) / 32,
-                               cudaMemcpyHostToDevice, stream));
+      if (int rc = upload_rows(st, stream, wsp + off_sa, static_cast<size_t>(m - 1) * d->ld_scales_a + (k + 31) / 32, d->a_scales, static_cast<size_t>(m - 1) * d->ld_scales_a + (k + 31) / 32, static_cast<size_t>(m - 1) * d->ld_scales_a + (k + 31) / 32, 1)) return rc;
       sa_ptr = wsp + off_sa;
     }
     if (is_mx && !sb_dev) {
-      CUDA_TRY(cudaMemcpyAsync(wsp + off_sb, d->b_scales, static_cast<size_t>(n - 1) * d->ld_scales_b + (k + 31) / 32,
-                               cudaMemcpyHostToDevice, stream));
+      if (int rc = upload_rows(st, stream, wsp + off_sb, static_cast<size_t>(n - 1) * d->ld_scales_b + (k + 31) / 32, d->b_scales, static_cast<size_t>(n - 1) * d->ld_scales_b + (k + 31) / 32, static_cast<size_t>(n - 1) * d->ld_scales_b + (k + 31) / 32, 1)) return rc;
       sb_ptr = wsp + off_sb;
     }
   }
   if (stage_c) {
-    CUDA_TRY(cudaMemcpy2DAsync(wsp + off_c, c_ld_dev * 4, d->c, static_cast<size_t>(d->ldc) * 4,
-                               c_inner * 4, c_outer, cudaMemcpyHostToDevice, stream));
+    if (int rc = upload_rows(st, stream, wsp + off_c, c_ld_dev * 4, d->c, static_cast<size_t>(d->ldc) * 4, c_inner * 4, c_outer)) return rc;
     c_ptr = wsp + off_c;
   } else if (!c_dev) {
     c_ptr = wsp;  // never dereferenced (beta == 0)
@@ -1443,8 +1442,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   }
 
   if (!d_dev) {
-    CUDA_TRY(cudaMemcpy2DAsync(d->d, static_cast<size_t>(d->ldd) * 4, d_ptr, d_ld_dev * 4, c_inner * 4,
-                               c_outer, cudaMemcpyDeviceToHost, stream));
+    if (int rc = download_rows(st, stream, d->d, static_cast<size_t>(d->ldd) * 4, d_ptr, d_ld_dev * 4, c_inner * 4, c_outer)) return rc;
   }
   if (async) return CPUOPS_B200_STATUS_SUCCESS;
 

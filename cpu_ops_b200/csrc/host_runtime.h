@@ -27,6 +27,7 @@
 #include "decode_kernel.cuh"
 #include "gemm_kernel.cuh"
 #include "gemm_params.h"
+#include "host_copy.h"
 
 namespace {
 
@@ -114,6 +115,7 @@ struct DeviceState {
   cudaStream_t panel_stream[kPanelStreams] = {nullptr, nullptr, nullptr};
   cudaEvent_t panel_done[kPanelStreams] = {nullptr, nullptr, nullptr};
   cudaEvent_t fork_event = nullptr;
+  StagingRing staging;  // pageable host operands (host_copy.h)
   // Largest number of two-CTA clusters of the pair kernel that can be resident at once,
   // per kind (-1: not asked yet; 0: cluster launch unavailable).
   int pair_clusters[3] = {-1, -1, -1};
@@ -274,8 +276,30 @@ int init_device(int device, DeviceState** out) {
   return 0;
 }
 
+// Host -> device and device -> host copies of `rows` rows of `width` bytes.  A download from
+// pageable memory is complete after st.staging.finish() (finish_stream calls it).
+int upload_rows(DeviceState& st, cudaStream_t stream, void* dst, size_t dst_pitch, const void* src, size_t src_pitch,
+                size_t width, size_t rows) {
+  if (st.staging.serves(src, width, width * rows, stream)) {
+    CUDA_TRY(st.staging.upload(dst, dst_pitch, src, src_pitch, width, rows, stream));
+  } else {
+    CUDA_TRY(cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, rows, cudaMemcpyHostToDevice, stream));
+  }
+  return 0;
+}
+int download_rows(DeviceState& st, cudaStream_t stream, void* dst, size_t dst_pitch, const void* src, size_t src_pitch,
+                  size_t width, size_t rows) {
+  if (st.staging.serves(dst, width, width * rows, stream)) {
+    CUDA_TRY(st.staging.download(dst, dst_pitch, src, src_pitch, width, rows, stream));
+  } else {
+    CUDA_TRY(cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, rows, cudaMemcpyDeviceToHost, stream));
+  }
+  return 0;
+}
+
 // Waits for the stream's work and reports (and clears) what its kernels left in the error word.
 int finish_stream(DeviceState& st, cudaStream_t stream) {
+  CUDA_TRY(st.staging.finish());  // downloads into pageable memory, as they arrive
   CUDA_TRY(cudaStreamSynchronize(stream));
   const int32_t code = *st.error_host;
   if (code == 0) return CPUOPS_B200_STATUS_SUCCESS;
