@@ -1293,6 +1293,9 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       // well before four warps have drained the previous tile (about 1500 cycles per
       // 32-column chunk each): measured +10-15 % at K = 1024, nothing at K = 2048
       if (2 * (k_blocks / ch.slices) <= 3 * (ch.BN / 32) && ch.BN >= 128) epi_warps = 8;
+      // ... or, C or D going through the ring by rows (twice the instructions per chunk), when
+      // k is short: 1999 x 3001 x 1777 (14 k-blocks, BN 128), four / eight warps 29.6 / 27.5 us
+      if ((p.c_ring == kRingRows || p.d_ring == kRingRows) && k_blocks <= 4 * (ch.BN / 32) && ch.BN >= 128) epi_warps = 8;
       // ... or when the chain holds a Gelu or Silu (about 20 instructions and two MUFU
       // operations per element) and the k loop is not long enough for four warps to issue
       // them behind it.  With bias + SiLU, four / eight warps: e4m3 2048 x 4096 x 2048 (16

@@ -25,6 +25,8 @@
 // for copies and MMAs still in flight before tensor memory is released.
 #pragma once
 
+#include <type_traits>
+
 #include "epilogue.cuh"
 #include "gemm_params.h"
 #include "ptx_sm100.cuh"
@@ -123,14 +125,14 @@ __device__ __forceinline__ void fetch_c_chunk(const GemmParams& p, uint32_t buf,
   const int nrows = p.Mk - row0, ncols = p.Nk - kcol0;  // what the matrix still has from here on
   if (p.c_ring == kRingRows) {
     const uint32_t* src = base + (lane < ncols ? lane : 0);
-#pragma unroll
+#pragma unroll 8  // (short: the code of the TMA paths around it stays close together)
     for (int r = 0; r < 32; ++r, src += e.c_sr) {
       const bool valid = r < nrows && lane < ncols;
       copy_word_async(buf + ring_word(r, lane), valid ? src : static_cast<const uint32_t*>(e.C), valid);
     }
   } else {
     const uint32_t* src = base + lane;
-#pragma unroll
+#pragma unroll 8
     for (int i = 0; i < 32; ++i, src += e.c_sc) {
       const bool valid = lane < nrows && i < ncols;
       copy_word_async(buf + static_cast<uint32_t>(i * 128 + lane * 4),
@@ -146,7 +148,7 @@ __device__ __forceinline__ void write_d_rows(const GemmParams& p, uint32_t buf, 
   const EpilogueParams& e = p.epi;
   uint32_t* dst = static_cast<uint32_t*>(e.D) + (row0 * e.d_sr + kcol0 + lane);
   const int nrows = lane < p.Nk - kcol0 ? p.Mk - row0 : 0;
-#pragma unroll
+#pragma unroll 1
   for (int r0 = 0; r0 < 32; r0 += 8) {
     uint32_t v[8];
 #pragma unroll
@@ -163,7 +165,7 @@ __device__ __forceinline__ void write_d_rows(const GemmParams& p, uint32_t buf, 
 // the ring, or 0 (kRingColumns: of the thread's first word, the next ones 128 bytes apart).
 // `d_smem_row`: where to put the finished row for the TMA store or write_d_rows, or 0
 // (store directly).  Explicit shared-space accesses: generic ones cost more.
-template <bool kInt>
+template <bool kInt, bool kTmaOnly>
 __device__ __forceinline__ void store_chunk(const GemmParams& p, uint32_t (&r)[32], int krow,
                                             int kcol0, int slice, uint32_t c_smem_row,
                                             uint32_t d_smem_row, int c_swz) {
@@ -183,7 +185,7 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, uint32_t (&r)[3
   }
   const EpilogueParams& e = p.epi;
   uint32_t src[32];
-  if (c_smem_row != 0 && p.c_ring == kRingColumns) {
+  if (!kTmaOnly && c_smem_row != 0 && p.c_ring == kRingColumns) {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
       asm volatile("ld.shared.u32 %0, [%1];" : "=r"(src[i]) : "r"(c_smem_row + 128u * i));
@@ -644,81 +646,69 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
     // A third buffer (p.ring_bufs == 3) hides that wait at the price of shared memory.
     // TMA carries what it can address; the rest goes through cp.async and plain stores
     // (fetch_c_chunk, write_d_rows): 1999 x 3001 x 1777 with leading dimensions of dim + 3
-    // and beta = 1, 36.8 -> 29.3 us (with the copy of A and B below).
-    const bool ring = p.c_ring != kRingNone, d_tma = p.d_ring == kRingTma, d_rows = p.d_ring == kRingRows;
-    const bool c_tma = p.c_ring == kRingTma;
-    const uint32_t nb = static_cast<uint32_t>(p.ring_bufs);
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // before C is read, D or a slab written
-    warm_epilogue_params(p.epi);  // constant-cache misses now, not after the first accumulator
-    asm volatile("" ::"r"(p.Mk ^ p.Nk ^ p.mode), "l"(p.ws), "l"(p.ws_slab ^ p.ws_sr ^ p.ws_sc));
-    const uint32_t my_c = c_base + static_cast<uint32_t>(ew) * nb * 4096u;
-    uint32_t cq = 0;        // chunks consumed so far by this warp
-    uint32_t cq_b = 0, cq_ph = 0;  // its buffer and that buffer's barrier parity
-    uint32_t cissued = 0, ci_b = 0;  // C chunks requested so far, buffer of the next request
-    bool alive = true;
-    const bool edbg = B200_CLK(p) != nullptr && blockIdx.x == 0 && warp == 2 && lane == 0;
-    long long edbg_wait = 0;
-    const long long edbg_start = edbg ? clock64() : 0;
-    // pair: the leader's MMA thread waits for the epilogue warps of both CTAs
-    const uint32_t acc_empty0 = kPair ? map_to_cta(acc_empty_bar(0), 0) : acc_empty_bar(0);
-    auto request_c = [&](int col, int row) {  // TMA: lane 0 only; otherwise the whole warp
-      if (c_tma) {
-        mbar_expect_tx(c_full_bar(ew, ci_b), 4096u);
-        tma_load_2d(my_c + ci_b * 4096u, &tmC, c_full_bar(ew, ci_b), col, row);
-      } else {
-        fetch_c_chunk(p, my_c + ci_b * 4096u, row, col, lane);
-      }
-      ++cissued;
-      if (++ci_b == nb) ci_b = 0;
-    };
-    for (int t = work0; t < total_tiles && alive; t += work_step, ++it) {
-      const TileCoord tc = decode_tile(p, t, work_step);
-      const int buf = it % nacc;
-      const uint32_t acc_ph = static_cast<uint32_t>(it / nacc) & 1u;
-      const int row0 = (tc.m_tile * kCtas + static_cast<int>(cta_rank)) * kTileM + q * 32;
-      const int krow = row0 + lane;
-      const int n0 = tc.n_tile * p.BN;
-      const int nchunks = tc.bn / 32;
-      if (ring && (lane == 0 || !c_tma)) {
-        // this warp's first two chunks of the tile: requested before the accumulator is ready
-        // (cp.async: always two groups, so that the count stays in step)
-        if (d_tma && lane == 0) bulk_wait_group_read<0>();
-        if (!c_tma) __syncwarp();
-        for (int c = c0; c < c0 + 2 * cstep; c += cstep) {
-          if (c < nchunks) request_c(n0 + c * 32, row0);
-          if (!c_tma) cp_async_commit();
+    // and beta = 1, 36.8 -> 28 us (with the copy of A and B below).
+    // That code is a second instance of the loop below: as branches inside one loop it cost the
+    // TMA paths 0.3 of 17.2 us (int8 2048^3).
+    auto run_epilogue = [&](auto tma_only) {
+      constexpr bool kTmaOnly = decltype(tma_only)::value;  // each of C and D by TMA or not through the ring
+      const bool ring = p.c_ring != kRingNone, d_tma = p.d_ring == kRingTma;
+      const bool c_tma = kTmaOnly ? ring : p.c_ring == kRingTma, d_rows = !kTmaOnly && p.d_ring == kRingRows;
+      const uint32_t nb = static_cast<uint32_t>(p.ring_bufs);
+      asm volatile("griddepcontrol.wait;" ::: "memory");  // before C is read, D or a slab written
+      warm_epilogue_params(p.epi);  // constant-cache misses now, not after the first accumulator
+      asm volatile("" ::"r"(p.Mk ^ p.Nk ^ p.mode), "l"(p.ws), "l"(p.ws_slab ^ p.ws_sr ^ p.ws_sc));
+      const uint32_t my_c = c_base + static_cast<uint32_t>(ew) * nb * 4096u;
+      uint32_t cq = 0;        // chunks consumed so far by this warp
+      uint32_t cq_b = 0, cq_ph = 0;  // its buffer and that buffer's barrier parity
+      uint32_t cissued = 0, ci_b = 0;  // C chunks requested so far, buffer of the next request
+      bool alive = true;
+      const bool edbg = B200_CLK(p) != nullptr && blockIdx.x == 0 && warp == 2 && lane == 0;
+      long long edbg_wait = 0;
+      const long long edbg_start = edbg ? clock64() : 0;
+      // pair: the leader's MMA thread waits for the epilogue warps of both CTAs
+      const uint32_t acc_empty0 = kPair ? map_to_cta(acc_empty_bar(0), 0) : acc_empty_bar(0);
+      auto request_c = [&](int col, int row) {  // TMA: lane 0 only; otherwise the whole warp
+        if (kTmaOnly || c_tma) {
+          mbar_expect_tx(c_full_bar(ew, ci_b), 4096u);
+          tma_load_2d(my_c + ci_b * 4096u, &tmC, c_full_bar(ew, ci_b), col, row);
+        } else {
+          fetch_c_chunk(p, my_c + ci_b * 4096u, row, col, lane);
         }
-      }
-      const long long te0 = edbg ? clock64() : 0;
-      const bool ready = mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
-      if (!__all_sync(0xffffffffu, ready)) {
-        if (lane == 0) record_error(p, abort_flag, kErrEpilogueWait);
-        alive = false;
-        break;
-      }
-      if (edbg) edbg_wait += clock64() - te0;
-      tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                             static_cast<uint32_t>(buf * p.BN);
-      if (c0 >= nchunks) {
-        // a tile narrower than this warp's first chunk: nothing to read, hand it back
-        tc_fence_before_sync();
-        if (lane == 0) {
-          if constexpr (kPair) {
-            mbar_arrive_cluster(acc_empty0 + 8u * buf);
-          } else {
-            mbar_arrive(acc_empty_bar(buf));
+        ++cissued;
+        if (++ci_b == nb) ci_b = 0;
+      };
+      for (int t = work0; t < total_tiles && alive; t += work_step, ++it) {
+        const TileCoord tc = decode_tile(p, t, work_step);
+        const int buf = it % nacc;
+        const uint32_t acc_ph = static_cast<uint32_t>(it / nacc) & 1u;
+        const int row0 = (tc.m_tile * kCtas + static_cast<int>(cta_rank)) * kTileM + q * 32;
+        const int krow = row0 + lane;
+        const int n0 = tc.n_tile * p.BN;
+        const int nchunks = tc.bn / 32;
+        if (ring && (lane == 0 || (!kTmaOnly && !c_tma))) {
+          // this warp's first two chunks of the tile: requested before the accumulator is ready
+          // (cp.async: always two groups, so that the count stays in step)
+          if (d_tma && lane == 0) bulk_wait_group_read<0>();
+          if (!kTmaOnly && !c_tma) __syncwarp();
+          for (int c = c0; c < c0 + 2 * cstep; c += cstep) {
+            if (c < nchunks) request_c(n0 + c * 32, row0);
+            if (!kTmaOnly && !c_tma) cp_async_commit();
           }
         }
-      }
-      for (int c = c0; c < nchunks; c += cstep) {
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + static_cast<uint32_t>(c * 32), r);
-        tmem_ld_wait();
-        if (c + cstep >= nchunks) {
-          // the accumulator is in registers: hand the buffer back to the MMA warp
+        const long long te0 = edbg ? clock64() : 0;
+        const bool ready = mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
+        if (!__all_sync(0xffffffffu, ready)) {
+          if (lane == 0) record_error(p, abort_flag, kErrEpilogueWait);
+          alive = false;
+          break;
+        }
+        if (edbg) edbg_wait += clock64() - te0;
+        tc_fence_after_sync();
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
+                               static_cast<uint32_t>(buf * p.BN);
+        if (c0 >= nchunks) {
+          // a tile narrower than this warp's first chunk: nothing to read, hand it back
           tc_fence_before_sync();
-          __syncwarp();
           if (lane == 0) {
             if constexpr (kPair) {
               mbar_arrive_cluster(acc_empty0 + 8u * buf);
@@ -727,87 +717,109 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
             }
           }
         }
-        const int kcol0 = n0 + c * 32;
-        uint32_t c_row = 0, d_row = 0;  // shared-memory addresses of this lane's row
-        if (ring && !c_tma) {
-          cp_async_wait<1>();  // all groups but the youngest: this chunk's
-          __syncwarp();        // ... of every lane
-          c_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * (p.c_ring == kRingColumns ? 4u : 128u);
-        } else if (ring) {
-          const bool got = mbar_wait_bounded(c_full_bar(ew, cq_b), cq_ph, abort_flag, budget_ns);
-          if (!__all_sync(0xffffffffu, got)) {
-            if (lane == 0) record_error(p, abort_flag, kErrEpilogueWait);
-            alive = false;
-            break;
-          }
-          c_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * 128u;
-        } else if (d_tma) {
-          // the store that last read this buffer (nb chunks ago) must be done with it
-          if (lane == 0) {
-            if (nb >= 3) bulk_wait_group_read<2>(); else bulk_wait_group_read<1>();
-          }
-          __syncwarp();
-        }
-        if (d_tma || d_rows) d_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * 128u;
-        if (krow < p.Mk && kcol0 < p.Nk)
-          store_chunk<kInt>(p, r, krow, kcol0, tc.slice, c_row, d_row, lane & 7);
-        if (d_tma) {
-          fence_proxy_async_shared_cta();  // this lane's row -> visible to the TMA store
-          __syncwarp();
-          if (lane == 0) {
-            if (row0 < p.Mk && kcol0 < p.Nk) tma_store_2d(&tmD, my_c + cq_b * 4096u, kcol0, row0);
-            bulk_commit_group();
-          }
-        } else if (d_rows) {
-          __syncwarp();  // every lane's row is there
-          write_d_rows(p, my_c + cq_b * 4096u, row0, kcol0, lane);
-          __syncwarp();  // every lane has read its words: the buffer may be written again
-        } else if (ring) {
-          __syncwarp();  // every lane has read its row: the buffer may be refilled
-        }
-        if (ring && c_tma && lane == 0 && c + 2 * cstep < nchunks) {
-          // chunk c + 2 goes where chunk c (two buffers) or chunk c - 1 (three) was: the
-          // store out of that buffer must have read it first.  With three buffers that is
-          // the store before the one just issued, which has normally finished by now.
-          if (d_tma) {
-            if (nb >= 3) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
-          }
-          request_c(n0 + (c + 2 * cstep) * 32, row0);
-        } else if (ring && !c_tma) {
-          if (c + 2 * cstep < nchunks) {
-            if (d_tma) {  // (as above; lane 0 holds the bulk groups)
-              if (lane == 0) {
-                if (nb >= 3) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
+        for (int c = c0; c < nchunks; c += cstep) {
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + static_cast<uint32_t>(c * 32), r);
+          tmem_ld_wait();
+          if (c + cstep >= nchunks) {
+            // the accumulator is in registers: hand the buffer back to the MMA warp
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+              if constexpr (kPair) {
+                mbar_arrive_cluster(acc_empty0 + 8u * buf);
+              } else {
+                mbar_arrive(acc_empty_bar(buf));
               }
-              __syncwarp();
+            }
+          }
+          const int kcol0 = n0 + c * 32;
+          uint32_t c_row = 0, d_row = 0;  // shared-memory addresses of this lane's row
+          if (!kTmaOnly && ring && !c_tma) {
+            cp_async_wait<1>();  // all groups but the youngest: this chunk's
+            __syncwarp();        // ... of every lane
+            c_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * (p.c_ring == kRingColumns ? 4u : 128u);
+          } else if (ring) {
+            const bool got = mbar_wait_bounded(c_full_bar(ew, cq_b), cq_ph, abort_flag, budget_ns);
+            if (!__all_sync(0xffffffffu, got)) {
+              if (lane == 0) record_error(p, abort_flag, kErrEpilogueWait);
+              alive = false;
+              break;
+            }
+            c_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * 128u;
+          } else if (d_tma) {
+            // the store that last read this buffer (nb chunks ago) must be done with it
+            if (lane == 0) {
+              if (nb >= 3) bulk_wait_group_read<2>(); else bulk_wait_group_read<1>();
+            }
+            __syncwarp();
+          }
+          if (d_tma || d_rows) d_row = my_c + cq_b * 4096u + static_cast<uint32_t>(lane) * 128u;
+          if (krow < p.Mk && kcol0 < p.Nk)
+            store_chunk<kInt, kTmaOnly>(p, r, krow, kcol0, tc.slice, c_row, d_row, lane & 7);
+          if (d_tma) {
+            fence_proxy_async_shared_cta();  // this lane's row -> visible to the TMA store
+            __syncwarp();
+            if (lane == 0) {
+              if (row0 < p.Mk && kcol0 < p.Nk) tma_store_2d(&tmD, my_c + cq_b * 4096u, kcol0, row0);
+              bulk_commit_group();
+            }
+          } else if (d_rows) {
+            __syncwarp();  // every lane's row is there
+            write_d_rows(p, my_c + cq_b * 4096u, row0, kcol0, lane);
+            __syncwarp();  // every lane has read its words: the buffer may be written again
+          } else if (ring) {
+            __syncwarp();  // every lane has read its row: the buffer may be refilled
+          }
+          if (ring && c_tma && lane == 0 && c + 2 * cstep < nchunks) {
+            // chunk c + 2 goes where chunk c (two buffers) or chunk c - 1 (three) was: the
+            // store out of that buffer must have read it first.  With three buffers that is
+            // the store before the one just issued, which has normally finished by now.
+            if (d_tma) {
+              if (nb >= 3) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
             }
             request_c(n0 + (c + 2 * cstep) * 32, row0);
+          } else if (!kTmaOnly && ring && !c_tma) {
+            if (c + 2 * cstep < nchunks) {
+              if (d_tma) {  // (as above; lane 0 holds the bulk groups)
+                if (lane == 0) {
+                  if (nb >= 3) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
+                }
+                __syncwarp();
+              }
+              request_c(n0 + (c + 2 * cstep) * 32, row0);
+            }
+            cp_async_commit();
           }
-          cp_async_commit();
-        }
-        ++cq;
-        if (++cq_b == nb) {
-          cq_b = 0;
-          cq_ph ^= 1u;
-        }
-      }
-    }
-    if (d_tma && lane == 0) bulk_wait_group_all();  // D is complete before the kernel ends
-    if (edbg) {
-      B200_CLK(p)[5] = static_cast<unsigned long long>(clock64() - edbg_start);
-      B200_CLK(p)[6] = static_cast<unsigned long long>(edbg_wait);
-    }
-    if (ring && !c_tma) cp_async_wait<0>();
-    if (c_tma && *abort_flag != 0 && lane == 0) {
-      // let C chunks that were requested but never consumed land before the CTA exits
-      int dummy = 0;
-      for (; cq < cissued; ++cq) {
-        mbar_wait_bounded(c_full_bar(ew, cq_b), cq_ph, &dummy, budget_ns);
-        if (++cq_b == nb) {
-          cq_b = 0;
-          cq_ph ^= 1u;
+          ++cq;
+          if (++cq_b == nb) {
+            cq_b = 0;
+            cq_ph ^= 1u;
+          }
         }
       }
+      if (d_tma && lane == 0) bulk_wait_group_all();  // D is complete before the kernel ends
+      if (edbg) {
+        B200_CLK(p)[5] = static_cast<unsigned long long>(clock64() - edbg_start);
+        B200_CLK(p)[6] = static_cast<unsigned long long>(edbg_wait);
+      }
+      if (!kTmaOnly && ring && !c_tma) cp_async_wait<0>();
+      if (c_tma && *abort_flag != 0 && lane == 0) {
+        // let C chunks that were requested but never consumed land before the CTA exits
+        int dummy = 0;
+        for (; cq < cissued; ++cq) {
+          mbar_wait_bounded(c_full_bar(ew, cq_b), cq_ph, &dummy, budget_ns);
+          if (++cq_b == nb) {
+            cq_b = 0;
+            cq_ph ^= 1u;
+          }
+        }
+      }
+    };
+    if (p.c_ring <= kRingTma && p.d_ring <= kRingTma) {
+      run_epilogue(std::true_type{});
+    } else {
+      run_epilogue(std::false_type{});
     }
   }
 
