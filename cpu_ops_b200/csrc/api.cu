@@ -88,6 +88,20 @@ bool pair_pays(int Mk, int Nk, int k_blocks, int BN, int slices, int sms, bool b
   return legal && tiles >= 2 * sms && k_blocks >= 8;
 }
 
+// The same for 256-wide tiles that all run at once (at most one per SM, unsplit).  A pair
+// starts and ends later than two CTAs (its barriers are remote), but stages 32 KB per k-block and
+// SM where a CTA stages 48 KB, so a long k loop wins.  One CTA per tile / pairs, both with
+// eight epilogue warps: u8 x s8 2048^3 beta = 1 (16 k-blocks) 17.3 / 16.8 us, beta = 0 14.2 / 14.5,
+// 1536 x 2816 x 1024 (8) 14.0 / 14.6, 1024 x 4096 x 4096 (32) 22.7 / 20.1, 2048 x 2304 x 8192
+// (64) 37.3 / 30.4; e4m3 2048^3 (16) 21.0 / 21.2, 1024 x 4096 x 4096 (32) 27.3 / 26.9,
+// 2048 x 2304 x 8192 (64) 47.2 / 43.7; e2m1 2048^3 (8) 17.4 / 18.0, 2048 x 2304 x 8192 (32)
+// 32.1 / 31.4.  At 16 k-blocks only the C that is read beside them decides.
+bool pair_pays_in_one_wave(int Mk, int Nk, int k_blocks, int BN, int sms, bool is_mx, bool beta) {
+  const int64_t pairs = static_cast<int64_t>((Mk + 255) / 256) * ((Nk + BN - 1) / BN);
+  const bool halves_full = (Mk + 127) / 128 % 2 == 0;
+  return BN == 256 && Mk > 128 && halves_full && 2 * pairs <= sms && k_blocks >= (!is_mx && beta ? 16 : 24);
+}
+
 // Estimated SM cycles of an unsplit launch with tile width BN.  Per k-block a CTA is bound
 // by the L2 -> shared-memory feed (about 64 bytes per cycle: 128 rows of A plus its rows of
 // B, 128 bytes each) or by the MMAs (BN / 2 cycles per 32-byte k step); the epilogue hides
@@ -821,7 +835,9 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     const int Mk = ch.swap ? n : m, Nk = ch.swap ? m : n;
     const bool bk_role_mn = !(ch.swap ? a_kmajor : b_kmajor);
     const bool legal = Mk > 128 && (!bk_role_mn || ch.BN == 256) && ch.BN % 32 == 0;
-    bool want = pair_pays(Mk, Nk, k_blocks, ch.BN, ch.slices, sms, bk_role_mn);
+    bool want = pair_pays(Mk, Nk, k_blocks, ch.BN, ch.slices, sms, bk_role_mn) ||
+                (ch.slices == 1 && d->tile_n == 0 &&
+                 pair_pays_in_one_wave(Mk, Nk, k_blocks, ch.BN, sms, is_mx, beta_nonzero));
     if (env_switches().pair >= 0) want = env_switches().pair != 0;
     if (d->flags & CPUOPS_B200_FLAG_PAIR_ON) want = true;
     if (d->flags & CPUOPS_B200_FLAG_PAIR_OFF) want = false;
@@ -1288,7 +1304,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     int epi_warps = 4;
     {
       const int64_t items = static_cast<int64_t>(p.m_tiles) * p.n_tiles * p.slices;
-      if (!ch.pair && items <= sms && ch.BN >= 128) epi_warps = 8;
+      if (items * (ch.pair ? 2 : 1) <= sms && ch.BN >= 128) epi_warps = 8;
       // ... or when k is so short that a tile's k loop (about 600 cycles per k-block) ends
       // well before four warps have drained the previous tile (about 1500 cycles per
       // 32-column chunk each): measured +10-15 % at K = 1024, nothing at K = 2048

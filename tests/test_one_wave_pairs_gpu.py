@@ -1,0 +1,28 @@
+"""256-wide tiles that all run at once go to CTA pairs when the k loop is long enough and no
+pair would be half empty; every choice gives the exact integer product."""
+import pytest
+import torch
+
+import cpu_ops_b200 as c
+from cpu_ops_b200 import _capi
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k,beta,pair", [
+    (2048, 2048, 2048, 1, 1), (2048, 2048, 2048, 0, 0), (2048, 2048, 1920, 1, 0), (1024, 4096, 4096, 0, 1),
+    (1000, 4090, 3200, 1, 1), (1024, 4096, 2944, 0, 0), (1100, 4096, 4096, 0, 0), (2048, 2304, 4096, 1, 1)])
+def test_pairs_in_one_wave(gpu, m, n, k, beta, pair):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    A = torch.randint(0, 256, (m, k), dtype=torch.uint8, device="cuda", generator=g)
+    B = torch.randint(-128, 128, (n, k), dtype=torch.int8, device="cuda", generator=g)
+    C = torch.randint(-1000, 1000, (m, n), dtype=torch.int32, device="cuda", generator=g)
+    D = torch.full((m, n), 77, dtype=torch.int32, device="cuda")
+    op = c.GemmU8S8S32(c.RowMajor, c.ColumnMajor, c.RowMajor)
+    st = op(op.Arguments(c.GemmCoord(m, n, k), c.TensorRef(A, k), c.TensorRef(B, k), c.TensorRef(C, n),
+                         c.TensorRef(D, n), c.LinearCombination(1, beta)))
+    assert st == c.Status.kSuccess, _capi.last_error()
+    if _capi.last_plan().tile_n == 256:
+        assert _capi.last_plan().pair == pair
+    # |sums| < 2^53: exact in f64
+    assert torch.equal(D, (A.double() @ B.double().T).to(torch.int32) + beta * C)
