@@ -96,10 +96,12 @@ bool pair_pays(int Mk, int Nk, int k_blocks, int BN, int slices, int sms, bool b
 // (64) 37.3 / 30.4; e4m3 2048^3 (16) 21.0 / 21.2, 1024 x 4096 x 4096 (32) 27.3 / 26.9,
 // 2048 x 2304 x 8192 (64) 47.2 / 43.7; e2m1 2048^3 (8) 17.4 / 18.0, 2048 x 2304 x 8192 (32)
 // 32.1 / 31.4.  At 16 k-blocks only the C that is read beside them decides.
-bool pair_pays_in_one_wave(int Mk, int Nk, int k_blocks, int BN, int sms, bool is_mx, bool beta) {
+// e2m1 has its raw scales in the one-CTA form only (kRaw), which is worth more: 25.6 us.
+bool pair_pays_in_one_wave(int Mk, int Nk, int k_blocks, int BN, int sms, int kind, bool beta) {
   const int64_t pairs = static_cast<int64_t>((Mk + 255) / 256) * ((Nk + BN - 1) / BN);
   const bool halves_full = (Mk + 127) / 128 % 2 == 0;
-  return BN == 256 && Mk > 128 && halves_full && 2 * pairs <= sms && k_blocks >= (!is_mx && beta ? 16 : 24);
+  return BN == 256 && Mk > 128 && halves_full && 2 * pairs <= sms && kind != kKindMxf4 &&
+         k_blocks >= (kind == kKindI8 && beta ? 16 : 24);
 }
 
 // Estimated SM cycles of an unsplit launch with tile width BN.  Per k-block a CTA is bound
@@ -837,7 +839,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     const bool legal = Mk > 128 && (!bk_role_mn || ch.BN == 256) && ch.BN % 32 == 0;
     bool want = pair_pays(Mk, Nk, k_blocks, ch.BN, ch.slices, sms, bk_role_mn) ||
                 (ch.slices == 1 && d->tile_n == 0 &&
-                 pair_pays_in_one_wave(Mk, Nk, k_blocks, ch.BN, sms, is_mx, beta_nonzero));
+                 pair_pays_in_one_wave(Mk, Nk, k_blocks, ch.BN, sms, kind, beta_nonzero));
     if (env_switches().pair >= 0) want = env_switches().pair != 0;
     if (d->flags & CPUOPS_B200_FLAG_PAIR_ON) want = true;
     if (d->flags & CPUOPS_B200_FLAG_PAIR_OFF) want = false;
@@ -848,14 +850,36 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   // (one launch, raw scales, every SM streaming an equal share of the weights).  It fetches the
   // scale rows 16 bytes at a time, which wants 16-byte aligned bases and leading dimensions; a
   // forced tile width or slice count keeps the general kernel, whose plan those describe.
+  auto scale_rows_aligned = [&](int to) {
+    auto aligned = [&](const void* ptr, bool on_device, int ld, int rows) {
+      return (!on_device || reinterpret_cast<uintptr_t>(ptr) % to == 0) && (rows <= 1 || ld % to == 0);
+    };
+    return aligned(d->a_scales, sa_dev, d->ld_scales_a, m) && aligned(d->b_scales, sb_dev, d->ld_scales_b, n);
+  };
   DecodePlan dp;
   if (k > 0 && is_mx && !mixed && ch.swap && m <= 64 && d->tile_n == 0 && d->split_k_slices <= 1 &&
       !(d->flags & (CPUOPS_B200_FLAG_PAIR_ON | CPUOPS_B200_FLAG_PAIR_OFF)) && !env_switches().no_decode) {
-    auto scales_ok = [](const void* ptr, bool on_device, int ld, int rows) {
-      return (!on_device || (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0) && (rows <= 1 || ld % 16 == 0);
-    };
-    if (scales_ok(d->a_scales, sa_dev, d->ld_scales_a, m) && scales_ok(d->b_scales, sb_dev, d->ld_scales_b, n))
-      dp = plan_decode(st, kind, n, m, k_blocks, d->split_k_slices == 1);
+    if (scale_rows_aligned(16)) dp = plan_decode(st, kind, n, m, k_blocks, d->split_k_slices == 1);
+  }
+
+  // ---- scales read by the GEMM kernel itself, or re-laid-out by a kernel in front of it -----------
+  // (kRaw in gemm_kernel.cuh.)  e2m1, whose k-block is 256 elements deep, gains in every launch of
+  // one CTA per tile.  e4m3 and e5m2 gain while the launch is short; over many k-blocks the
+  // longer way to a full stage costs more than the re-layout: e4m3 re-laid-out / raw, k-blocks
+  // that a CTA runs through: 4500 x 4500 x 640 (26) 37.4 / 34.0 us, 2048 x 3072 x 2048 (28) 23.7 / 22.2,
+  // 8192 x 4096 x 512 (33) 44.8 / 46, 2304 x 2304 x 4096 (58) 29.2 / 32.1, and with split k 128 x 8192 x
+  // 4096 27.5 / 28.7.  One tile per CTA hides more: 1100 x 4096 x 4096 (32) 31.1 / 25.4, 256 x 8192 x
+  // 8192 (64) 36.6 / 31.3.  A k-block's words must be aligned in every row: four bytes, e2m1 eight.
+  bool raw_scales = false;
+  if (is_mx && k > 0 && !mixed && !dp.use && !ch.pair && scale_rows_aligned(fp4_pair ? 8 : 4)) {
+    const int Mk = ch.swap ? n : m, Nk = ch.swap ? m : n;
+    const int64_t items = static_cast<int64_t>((Mk + 127) / 128) * ((Nk + ch.BN - 1) / ch.BN);
+    raw_scales = fp4_pair || (ch.slices == 1 && (items <= sms || items * k_blocks <= 32 * static_cast<int64_t>(sms)));
+  }
+  if (env_switches().raw >= 0) raw_scales = raw_scales && env_switches().raw != 0;
+  if (raw_scales && sb_dev) {
+    std::lock_guard<std::mutex> registry_lock(g_registry_mu);
+    if (find_prepared(st.device, d->b_scales, n, k, d->ld_scales_b)) raw_scales = false;
   }
 
   if (depth == 0 && k > 0 && !a_dev && !d_dev && !ch.swap && ch.slices == 1 && m >= 1024)
@@ -925,8 +949,10 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       sfa_bytes = cpuops_b200_scale_layout_bytes(ch.pair ? static_cast<int>(align_up(Mk, 256)) : Mk, k,
                                                  kTileM, bps);
       sfb_bytes = cpuops_b200_scale_layout_bytes(Nk, k, ch.BN, bps);
-      off_sfa = plan.take(sfa_bytes);
-      off_sfb = plan.take(sfb_bytes);
+      if (!raw_scales) {
+        off_sfa = plan.take(sfa_bytes);
+        off_sfb = plan.take(sfb_bytes);
+      }
     }
     if (ch.slices > 1 && !dp.use) off_ws = plan.take(static_cast<size_t>(ch.slices) * Mk * Nk * 4);
   }
@@ -1133,7 +1159,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     const int64_t bk_pitch = swap ? a_pitch_dev : b_pitch_dev;
     const bool ak_kmajor = swap ? b_kmajor : a_kmajor;
     const bool bk_kmajor = swap ? a_kmajor : b_kmajor;
-    if (is_mx) {
+    if (is_mx && !raw_scales) {
       const uint8_t* sak = swap ? sb_ptr : sa_ptr;
       const uint8_t* sbk = swap ? sa_ptr : sb_ptr;
       const int ldsak = swap ? d->ld_scales_b : d->ld_scales_a;
@@ -1263,6 +1289,11 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     if (is_mx) {
       p.sfa = sfa_dev;
       p.sfb = sfb_dev;
+      p.raw_a = swap ? sb_ptr : sa_ptr;
+      p.raw_b = swap ? sa_ptr : sb_ptr;
+      p.ld_raw_a = swap ? d->ld_scales_b : d->ld_scales_a;
+      p.ld_raw_b = swap ? d->ld_scales_a : d->ld_scales_b;
+      p.kblocks32 = (k + 31) / 32;
       p.sfa_stage_bytes = (bps / 4) * 512;
       p.sfb_stage_bytes = (bps / 4) * ((ch.BN + 127) / 128) * 512;
       const int sf_cols = (p.sfa_stage_bytes + p.sfb_stage_bytes) / 512 * 4;
@@ -1352,8 +1383,9 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     const int64_t total_tiles = static_cast<int64_t>(p.m_tiles) * p.n_tiles * p.slices;
     unsigned grid = static_cast<unsigned>(std::min<int64_t>(total_tiles, sms));
     CUtensorMap tmSFA = tmA, tmSFB = tmA;  // used by the pair kernel's scale loads only
+    const GemmKernel kernel = gemm_kernel(kind, ch.pair, raw_scales);
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(epi_warps == 8 ? kGemmThreadsWide : kGemmThreads);
+    cfg.blockDim = dim3((epi_warps == 8 ? kGemmThreadsWide : kGemmThreads) + (raw_scales ? 32 * kScaleWriterWarps : 0));
     cfg.dynamicSmemBytes = static_cast<size_t>(smem);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -1371,14 +1403,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
         probe.attrs = attr;
         probe.numAttrs = 1;
         int nc = 0;
-        cudaError_t e = cudaSuccess;
-        if (kind == kKindI8) {
-          e = cudaOccupancyMaxActiveClusters(&nc, gemm_tcgen05_kernel<kKindI8, true>, &probe);
-        } else if (kind == kKindMxf8) {
-          e = cudaOccupancyMaxActiveClusters(&nc, gemm_tcgen05_kernel<kKindMxf8, true>, &probe);
-        } else {
-          e = cudaOccupancyMaxActiveClusters(&nc, gemm_tcgen05_kernel<kKindMxf4, true>, &probe);
-        }
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&nc, kernel, &probe);
         if (e != cudaSuccess) {
           cudaGetLastError();
           nc = 0;
@@ -1391,7 +1416,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       }
       grid = 2u * static_cast<unsigned>(
                       std::min<int64_t>({total_tiles, static_cast<int64_t>(st.pair_clusters[kind]), sms / 2}));
-      if (is_mx) {
+      if (is_mx && !raw_scales) {
         if (int rc = make_tensor_map_atoms(&tmSFA, p.sfa, sfa_bytes / 512, p.sfa_stage_bytes / 512)) return rc;
         if (int rc = make_tensor_map_atoms(&tmSFB, p.sfb, sfb_bytes / 512, p.sfb_stage_bytes / 512)) return rc;
       }
@@ -1427,25 +1452,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     g_last_plan.narrow_last = p.narrow_last;
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
-    if (kind == kKindI8) {
-      if (ch.pair) {
-        CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kKindI8, true>, tmA, tmB, tmC, tmD, tmSFA, tmSFB, p));
-      } else {
-        CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kKindI8, false>, tmA, tmB, tmC, tmD, tmSFA, tmSFB, p));
-      }
-    } else if (kind == kKindMxf8) {
-      if (ch.pair) {
-        CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kKindMxf8, true>, tmA, tmB, tmC, tmD, tmSFA, tmSFB, p));
-      } else {
-        CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kKindMxf8, false>, tmA, tmB, tmC, tmD, tmSFA, tmSFB, p));
-      }
-    } else {
-      if (ch.pair) {
-        CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kKindMxf4, true>, tmA, tmB, tmC, tmD, tmSFA, tmSFB, p));
-      } else {
-        CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<kKindMxf4, false>, tmA, tmB, tmC, tmD, tmSFA, tmSFB, p));
-      }
-    }
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, tmC, tmD, tmSFA, tmSFB, p));
     g_launches.fetch_add(1);
     CUDA_TRY(cudaGetLastError());
     if (profile) {

@@ -44,6 +44,7 @@ namespace b200 {
 
 constexpr int kGemmThreads = 224;      // producer, MMA issuer, 4 epilogue warps, second producer
 constexpr int kGemmThreadsWide = 352;  // ... or 8 epilogue warps, two per TMEM lane quarter
+constexpr int kScaleWriterWarps = 4;   // kRaw: four more, which turn raw scales into atoms
 constexpr uint32_t kTmemCols = 512;
 
 struct TileCoord {
@@ -238,14 +239,131 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, uint32_t (&r)[3
   }
 }
 
+// The scale writers of the kRaw kernels.  Writer warp w makes the atoms of every k-block whose
+// running number is w modulo the number of writers: lane l reads the scale words (four or eight
+// blocks) of the rows l + 32 j of the tile's A and B scales and stores, per atom, the 16 bytes at
+// 16 l, which hold the words of four of those rows.  (All four warps on every k-block, a quarter
+// of the rows each, is a chain of latencies per k-block - the free stage, the stores, the proxy
+// fence, the arrival - that one k-block's MMAs do not cover: e4m3 512 x 2048 x 1024 11.5 us, 8.8 in
+// this form.)
+// Rows and k blocks outside the matrix get 127 (scale 1.0; the operand data there is zero)
+// and are never read.
+template <int KIND>
+__device__ __forceinline__ void write_scale_atoms(const GemmParams& p, int writer, int lane, uint32_t sf_base,
+                                                  int sf_stage, uint32_t full0, uint32_t empty0, int work0,
+                                                  int work_step, int total_tiles, volatile int* abort_flag,
+                                                  uint64_t budget_ns) {
+  constexpr int kKa = KIND == kKindMxf4 ? 2 : 1;  // scale words per row and k-block
+  const int stages = p.stages, nb128 = (p.BN + 127) / 128;
+  // No more writers than stages: a writer has seen the k-block `writers + stages` before its next
+  // one consumed, which must be no earlier than the last but one use of that next one's stage -
+  // a barrier's parity tells only two neighbouring uses apart.
+  const int writers = min(kScaleWriterWarps, stages);
+  if (writer >= writers) return;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // read cursor: this warp's next k-block to request
+  int f_t = work0, f_kb = 0, f_end = 0;
+  const uint8_t* row_a = nullptr;  // this lane's first row of the cursor's tile (and of its B scales)
+  const uint8_t* row_b = nullptr;
+  int rows_a = 0, rows_b = 0;      // how many rows exist from there on
+  auto enter_tile = [&](int skip) {  // `skip` k-blocks into the cursor's tile, or a later one
+    while (f_t < total_tiles) {
+      const TileCoord tc = decode_tile(p, f_t, work_step);
+      if (skip < tc.nkb) {
+        f_kb = tc.kb0 + skip;
+        f_end = tc.kb0 + tc.nkb;
+        const int ra = tc.m_tile * kTileM + lane, rb = tc.n_tile * p.BN + lane;
+        row_a = p.raw_a + static_cast<int64_t>(ra) * p.ld_raw_a;
+        row_b = p.raw_b + static_cast<int64_t>(rb) * p.ld_raw_b;
+        rows_a = p.Mk - ra;
+        rows_b = min(p.Nk - rb, p.BN - lane);
+        return;
+      }
+      skip -= tc.nkb;
+      f_t += work_step;
+    }
+  };
+  auto read_word = [&](const uint8_t* row, bool exists, uint32_t (&w)[kKa]) {
+#pragma unroll
+    for (int a = 0; a < kKa; ++a) w[a] = 0x7F7F7F7Fu;
+    if (!exists) return;
+    const int col = f_kb * 4 * kKa;
+    if (col + 4 * kKa <= p.kblocks32) {
+      if constexpr (kKa == 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(row + col);
+        w[0] = v.x;
+        w[1] = v.y;
+      } else {
+        w[0] = *reinterpret_cast<const uint32_t*>(row + col);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4 * kKa; ++i)
+        if (col + i < p.kblocks32)
+          w[i >> 2] = (w[i >> 2] & ~(0xFFu << (8 * (i & 3)))) | (static_cast<uint32_t>(row[col + i]) << (8 * (i & 3)));
+    }
+  };
+  uint32_t va[4][kKa], vb[8][kKa];
+  auto read_block = [&]() {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) read_word(row_a + static_cast<int64_t>(32 * j) * p.ld_raw_a, 32 * j < rows_a, va[j]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) read_word(row_b + static_cast<int64_t>(32 * j) * p.ld_raw_b, 32 * j < rows_b, vb[j]);
+    f_kb += writers;
+    if (f_kb >= f_end) {
+      const int skip = f_kb - f_end;
+      f_t += work_step;
+      enter_tile(skip);
+    }
+  };
+  auto store_atom = [&](uint32_t dst, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+  };
+  enter_tile(writer);
+  int s = writer;
+  uint32_t ph = 0;
+  while (f_t < total_tiles) {
+    read_block();  // (in flight until the stage is free)
+    // the stage's previous atoms have been copied to tensor memory (its MMAs are done)
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(empty0 + 8u * s, ph ^ 1u, abort_flag, budget_ns))) {
+      if (lane == 0) record_error(p, abort_flag, kErrProducerWait);
+      return;
+    }
+    const uint32_t dst = sf_base + static_cast<uint32_t>(s * sf_stage) + 16u * static_cast<uint32_t>(lane);
+#pragma unroll
+    for (int a = 0; a < kKa; ++a) {
+      store_atom(dst + 512u * a, va[0][a], va[1][a], va[2][a], va[3][a]);
+      const uint32_t b = dst + static_cast<uint32_t>(kKa + a * nb128) * 512u;
+      store_atom(b, vb[0][a], vb[1][a], vb[2][a], vb[3][a]);
+      if (nb128 > 1) store_atom(b + 512u, vb[4][a], vb[5][a], vb[6][a], vb[7][a]);
+    }
+    fence_proxy_async_shared_cta();  // these words -> visible to tcgen05.cp
+    __syncwarp();
+    if (lane == 0) mbar_arrive(full0 + 8u * s);
+    s += writers;
+    if (s >= stages) {
+      s -= stages;
+      ph ^= 1u;
+    }
+  }
+}
+
 // kPair: launched as clusters of two CTAs; the pair computes 256-row tiles with the
 // cta_group::2 instructions (see ptx_sm100_pair.cuh).  CTA rank r of a pair stages
 // rows [128 r, 128 r + 128) of the A tile and rows [r BN/2, (r + 1) BN/2) of the B
 // tile, all loads credit the leader's full barrier, the leader's MMA thread frees the
 // stage in both CTAs with a multicast commit, and each CTA's epilogue warps drain their
 // own 128 accumulator rows.  p.m_tiles counts 256-row tiles in that case.
-template <int KIND, bool kPair>
-__global__ void __launch_bounds__(kGemmThreadsWide, 1)
+//
+// kRaw (MX, one CTA per tile): the scale factors come from the caller's row-major arrays.  Four
+// more warps read them and write each k-block's 512-byte atoms into its stage, where TMA
+// otherwise puts them from the copy that relayout_scales_kernel made.  That kernel, its launch
+// and the boundary behind it are what this saves; the price is a read of the scales per
+// tile instead of one in all, and a longer way from a free stage to a full one.  Re-laid-out /
+// raw: e4m3 512 x 2048 x 1024 12.8 / 8.8 us, 2048^3 17.9 / 15.4, 256 x 8192 x 8192 36.6 / 31.3; e2m1
+// 512 x 2048 x 1024 14.1 / 9.0, 1024 x 4096 x 4096 22.7 / 18.1, 2048 x 2304 x 8192 31.8 / 25.6.
+template <int KIND, bool kPair, bool kRaw = false>
+__global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWarps : 0), 1)
     gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                         const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmC,
@@ -254,6 +372,7 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
                         const __grid_constant__ CUtensorMap tmSFB, const GemmParams p) {
   constexpr bool kInt = (KIND == kKindI8);
   constexpr bool kMx = !kInt;
+  static_assert(!kRaw || (kMx && !kPair), "raw scales: MX operands, one CTA per tile");
   constexpr int kCtas = kPair ? 2 : 1;
   // Programmatic dependent launch: the next kernel in the stream may become resident as
   // this one's CTAs retire; in return every role of this kernel that touches global memory
@@ -284,8 +403,8 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
   const uint32_t c_base = (sf_base + stages * sf_stage + 1023u) & ~1023u;
   // Epilogue warps: 4, or 8 when launched with kGemmThreadsWide threads (two per TMEM lane
   // quarter, which take alternate 32-column chunks of the tile).
-  const int n_epi = static_cast<int>(blockDim.x >> 5) - 3;
-  const int warp_producer2 = 2 + n_epi;  // the last warp
+  const int n_epi = static_cast<int>(blockDim.x >> 5) - 3 - (kRaw ? kScaleWriterWarps : 0);
+  const int warp_producer2 = 2 + n_epi;  // the last warp (kRaw: the scale writers follow)
   const uint32_t bar_base =
       p.ring_bufs ? c_base + ring_bytes(p.ring_bufs, n_epi) : sf_base + stages * sf_stage;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
@@ -304,12 +423,14 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
   // and warp 0 fetches descriptors.
   if (warp == 2) {
     for (int i = lane; i < kBarriers; i += 32) {
-      // full: the producer's arrive.expect_tx; empty / accumulator full / drain: one
-      // tcgen05.commit; accumulator empty: one arrival per epilogue warp (of both CTAs);
-      // C chunk: the TMA load's expect_tx
+      // full: the producer's arrive.expect_tx (kRaw: and the arrival of a
+      // scale writer); empty / accumulator full / drain: one tcgen05.commit; accumulator
+      // empty: one arrival per epilogue warp (of both CTAs); C chunk: the TMA load's expect_tx
       const bool acc_empty = i == 2 * kMaxStages + 2 || i == 2 * kMaxStages + 3;
-      mbar_init(bar_base + 8u * static_cast<uint32_t>(i),
-                acc_empty ? static_cast<uint32_t>(n_epi) * kCtas : 1u);
+      uint32_t count = 1u;
+      if (kRaw && i < kMaxStages) count = 2u;
+      if (acc_empty) count = static_cast<uint32_t>(n_epi) * kCtas;
+      mbar_init(bar_base + 8u * static_cast<uint32_t>(i), count);
     }
     if (lane == 0) *abort_flag = 0;
     if constexpr (kPair) {
@@ -381,7 +502,7 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
       bool ok = true;
       // (a packed 4-bit operand of a mixed-format GEMM credits only its 64 data bytes per
       // 128-byte shared-memory row, so the count comes from the launcher)
-      const uint32_t tx_bytes = static_cast<uint32_t>(p.tx_operand_bytes + sf_stage);
+      const uint32_t tx_bytes = static_cast<uint32_t>(p.tx_operand_bytes + (kRaw ? 0 : sf_stage));
       // pair: every load of both CTAs credits the leader's barrier, which alone is armed
       // (by the leader's producer) with the bytes of both
       const uint32_t full0 = kPair ? map_to_cta(full_bar(0), 0) : full_bar(0), empty0 = empty_bar(0);
@@ -402,7 +523,7 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
         const int n0 = tc.n_tile * p.BN + static_cast<int>(cta_rank) * (tc.bn / kCtas);
         const uint8_t* sfa_base = nullptr;  // this tile's scale atoms, k-block 0
         const uint8_t* sfb_base = nullptr;
-        if constexpr (kMx) {
+        if constexpr (kMx && !kRaw) {
           sfa_base = p.sfa + static_cast<int64_t>(m_tile128) * p.k_blocks * p.sfa_stage_bytes;
           sfb_base = p.sfb + static_cast<int64_t>(tc.n_tile) * p.k_blocks * p.sfb_stage_bytes;
         }
@@ -445,7 +566,7 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
             for (int c = 0; c < b_chunks; ++c)
               tma_load_2d_g<kPair>(b_dst + c * 16384, &tmB, full_addr, n0 + c * 128, kx, el);
           }
-          if constexpr (kMx) {
+          if constexpr (kMx && !kRaw) {
             const int kb = tc.kb0 + i;
             if constexpr (kPair) {
               // rows of 512 bytes (one atom each) of the re-laid-out scale arrays
@@ -471,9 +592,14 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
       if (*abort_flag != 0 && el) {
         // Let copies that were already issued land before the CTA exits.
         int dummy = 0;
-        for (int st = 0; st < stages; ++st)
-          if (armed & (1u << st)) mbar_wait_bounded(full_bar(st), (armed_parity >> st) & 1u, &dummy, budget_ns);
-        if constexpr (kPair) {
+        if (!kRaw)
+          for (int st = 0; st < stages; ++st)
+            if (armed & (1u << st)) mbar_wait_bounded(full_bar(st), (armed_parity >> st) & 1u, &dummy, budget_ns);
+        if constexpr (kRaw) {
+          // (the full barriers also count the scale writers, which may have given up)
+          const uint64_t t_end = global_timer_ns() + 200000;
+          while (global_timer_ns() < t_end) __nanosleep(1000);
+        } else if constexpr (kPair) {
           // the peer cannot watch the leader's barriers: give its copies time to land
           if (!leader) {
             const uint64_t t_end = global_timer_ns() + 100000;
@@ -630,6 +756,11 @@ __global__ void __launch_bounds__(kGemmThreadsWide, 1)
       }
     }
     __syncwarp();
+  } else if (kRaw && warp > warp_producer2) {
+    // ------------------------------ scale writers ------------------------------
+    if constexpr (kRaw)
+      write_scale_atoms<KIND>(p, warp - warp_producer2 - 1, lane, sf_base, sf_stage, full_bar(0), empty_bar(0), work0,
+                              work_step, total_tiles, abort_flag, budget_ns);
   } else {
     // -------------------------------- epilogue --------------------------------
     // (warps 2 .. 2 + n_epi - 1; the second producer warp took the first branch)

@@ -80,6 +80,10 @@ struct GemmParams {
   const uint8_t* sfa;
   const uint8_t* sfb;
   int32_t sfa_stage_bytes, sfb_stage_bytes;  // per k-block
+  // ... or (kRaw kernels) the caller's scale arrays: rows of kblocks32 bytes, each aligned to a k-block's scale words
+  const uint8_t* raw_a;
+  const uint8_t* raw_b;
+  int32_t ld_raw_a, ld_raw_b, kblocks32;
   int32_t c_ring;           // kRing*: how C chunks are prefetched into a shared-memory ring
   int32_t d_ring;           // kRing*: how D chunks leave through that ring
   int32_t ring_bufs;        // ring buffers per epilogue warp: 0 (no ring) or 2

@@ -160,6 +160,18 @@ PreparedB* find_prepared(int device, const void* scales, int n, int k, int ld_sc
   return nullptr;
 }
 
+// The GEMM kernel's instantiations (raw scales: MX, no pairs).
+using GemmKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
+GemmKernel gemm_kernel(int kind, bool pair, bool raw_scales) {
+  if (kind == kKindI8) return pair ? gemm_tcgen05_kernel<kKindI8, true> : gemm_tcgen05_kernel<kKindI8, false>;
+  if (kind == kKindMxf8) {
+    if (raw_scales) return gemm_tcgen05_kernel<kKindMxf8, false, true>;
+    return pair ? gemm_tcgen05_kernel<kKindMxf8, true> : gemm_tcgen05_kernel<kKindMxf8, false>;
+  }
+  if (raw_scales) return gemm_tcgen05_kernel<kKindMxf4, false, true>;
+  return pair ? gemm_tcgen05_kernel<kKindMxf4, true> : gemm_tcgen05_kernel<kKindMxf4, false>;
+}
+
 DeviceState g_dev[64];
 EncodeTiledFn g_encode = nullptr;
 int g_device_count = -2;  // -2: not probed; guarded by g_registry_mu
@@ -253,18 +265,10 @@ int init_device(int device, DeviceState** out) {
         }
         g_encode = reinterpret_cast<EncodeTiledFn>(fn);
       }
-      CUDA_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<kKindI8, false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
-      CUDA_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<kKindMxf8, false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
-      CUDA_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<kKindMxf4, false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
-      CUDA_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<kKindI8, true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
-      CUDA_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<kKindMxf8, true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
-      CUDA_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<kKindMxf4, true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
+      for (int kind : {kKindI8, kKindMxf8, kKindMxf4})
+        for (int form = 0; form < 3; ++form)
+          CUDA_TRY(cudaFuncSetAttribute(gemm_kernel(kind, form == 1, form == 2),
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
       CUDA_TRY(cudaFuncSetAttribute(decode_mx_kernel<kKindMxf8>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
       CUDA_TRY(cudaFuncSetAttribute(decode_mx_kernel<kKindMxf4>,
@@ -374,10 +378,11 @@ struct EnvSwitches {
   int decode_splits = geti("CPUOPS_B200_DECODE_SPLITS", 0);
   int decode_stages = geti("CPUOPS_B200_DECODE_STAGES", 0);
   int producers = geti("CPUOPS_B200_PRODUCERS", 0);
+  int raw = geti("CPUOPS_B200_RAW", -1);              // -1: heuristic
 #else
   static constexpr bool no_c_ring = false, no_d_tma = false, clk = false, no_narrow = false,
                         no_decode = false, no_pdl = false;
-  static constexpr int panels = 0, raster_m = 0, pair = -1, ring = 0, epi_warps = 0, decode_splits = 0,
+  static constexpr int panels = 0, raster_m = 0, pair = -1, raw = -1, ring = 0, epi_warps = 0, decode_splits = 0,
                        decode_stages = 0, producers = 0;
 #endif
 };
