@@ -4,7 +4,8 @@
 // a download holds the calling thread until it is complete: 1024^3 u8 x s8 with beta = 1
 // (6 MB up, 4 MB down) took 720 us.  Here a few threads share each piece's copy into
 // (or out of) a ring of pinned slots, the bus transfers of the pieces before it run meanwhile, and a
-// download's last copy is left until the call has issued everything else: 357 us.
+// download's last copy is left until the call has issued everything else: 410 us (five threads 390, but
+// then one of them more often has no core when its piece is waited for).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -39,79 +40,92 @@ struct RowCopy {
   }
 };
 
-// A few threads that share one copy at a time with the thread that asks for it.  They are
-// started by the first large copy of the process, watch for the next copy for 200 us after each
-// (a call's pieces follow one another within microseconds), sleep otherwise, and end with the process
-// (detached: nothing joins them, in a forked child neither).
-// A caller that finds them busy with another caller's copy does its own alone.
+// A few threads that share one copy at a time with the thread that asks for it, in pieces of
+// about 64 KB that each of them takes when it is free: a thread that gets no core (torch's own
+// threads may be spinning on them all) delays nobody, where equal shares made calls wait a
+// scheduler's slice of 4 ms for it.  The threads are started by the first large copy of the
+// process, watch for the next copy for 200 us after each (a call's pieces follow one another
+// within microseconds), sleep otherwise, and end with the process (detached: nothing joins
+// them, in a forked child neither).  A caller that finds them busy with another caller's copy
+// does its own alone.
 class CopyThreads {
  public:
-  static constexpr int kThreads = 5;
+  static constexpr int kThreads = 3;
 
   void copy(const RowCopy& c) {
+    const size_t bytes = c.width * c.rows;
     std::unique_lock<std::mutex> mine(owner_mu_, std::defer_lock);
-    if (c.width * c.rows < (64u << 10) || !mine.try_lock()) {
+    if (bytes < (128u << 10) || !mine.try_lock()) {
       c.share(0, 1);
       return;
     }
     if (!started_) start();
+    const uint32_t parts = static_cast<uint32_t>(std::min<size_t>(1024, (bytes + (64u << 10) - 1) / (64u << 10)));
     job_ = c;
-    parts_ = n_threads_ + 1;
-    pending_.store(static_cast<int>(n_threads_), std::memory_order_relaxed);
-    {
-      std::lock_guard<std::mutex> lk(sleep_mu_);  // no sleeper misses the new number
-      job_number_.fetch_add(1, std::memory_order_release);
-    }
+    done_.store(0, std::memory_order_relaxed);
+    ticket_.store(make_ticket(++job_number_, parts, 0));  // (a sleeper that misses this only helps less)
     if (sleepers_.load() > 0) wake_.notify_all();
-    c.share(0, parts_);
-    while (pending_.load(std::memory_order_acquire) > 0) _mm_pause();
+    while (take_part()) {
+    }
+    while (done_.load(std::memory_order_acquire) < parts) _mm_pause();
   }
 
  private:
+  // The job's number (so that a late thread cannot take a part of one job for another's), how
+  // many parts it has, and the next one to be taken.
+  static uint64_t make_ticket(uint32_t number, uint32_t parts, uint32_t next) {
+    return static_cast<uint64_t>(number) << 32 | parts << 16 | next;
+  }
+  static bool has_work(uint64_t t) { return (t & 0xFFFF) < (t >> 16 & 0xFFFF); }
+
+  // Takes and copies one part; false when none is left.  While a part is being copied its job
+  // cannot end, so job_ is the ticket's.
+  bool take_part() {
+    uint64_t t = ticket_.load(std::memory_order_acquire);
+    do {
+      if (!has_work(t)) return false;
+    } while (!ticket_.compare_exchange_weak(t, t + 1, std::memory_order_acq_rel, std::memory_order_acquire));
+    job_.share(t & 0xFFFF, t >> 16 & 0xFFFF);
+    done_.fetch_add(1, std::memory_order_release);
+    return true;
+  }
+
   void start() {
     started_ = true;
     const unsigned cores = std::thread::hardware_concurrency();
     const int n = std::max(0, std::min(kThreads, static_cast<int>(cores) / 2 - 1));
     try {
-      for (int i = 0; i < n; ++i) {
-        std::thread([this, i] { run(static_cast<size_t>(i) + 1); }).detach();
-        ++n_threads_;
-      }
+      for (int i = 0; i < n; ++i) std::thread([this] { run(); }).detach();
     } catch (...) {
       // no more threads to be had: the ones that exist share the work
     }
   }
 
-  void run(size_t part) {
-    uint64_t seen = 0;
+  void run() {
     for (;;) {
       const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
-      uint64_t now = job_number_.load(std::memory_order_acquire);
-      for (int i = 0; now == seen; ++i) {
+      bool found = false;
+      for (int i = 0; !found; ++i) {
+        found = take_part();
+        if (found) break;
         _mm_pause();
-        now = job_number_.load(std::memory_order_acquire);
         if ((i & 63) == 63 && std::chrono::steady_clock::now() > until) break;
       }
-      if (now == seen) {
-        std::unique_lock<std::mutex> lk(sleep_mu_);
-        sleepers_.fetch_add(1);
-        wake_.wait(lk, [&] { return job_number_.load() != seen; });
-        sleepers_.fetch_sub(1);
-        continue;
-      }
-      seen = now;
-      job_.share(part, parts_);
-      pending_.fetch_sub(1, std::memory_order_release);
+      if (found) continue;
+      std::unique_lock<std::mutex> lk(sleep_mu_);
+      sleepers_.fetch_add(1);
+      wake_.wait(lk, [&] { return has_work(ticket_.load()); });
+      sleepers_.fetch_sub(1);
     }
   }
 
   std::mutex owner_mu_;  // held by the caller whose copy is being shared
   bool started_ = false;
-  size_t n_threads_ = 0;
   RowCopy job_{};
-  size_t parts_ = 1;
-  std::atomic<uint64_t> job_number_{0};
-  std::atomic<int> pending_{0}, sleepers_{0};
+  uint32_t job_number_ = 0;
+  std::atomic<uint64_t> ticket_{0};
+  std::atomic<uint32_t> done_{0};
+  std::atomic<int> sleepers_{0};
   std::mutex sleep_mu_;
   std::condition_variable wake_;
 };
