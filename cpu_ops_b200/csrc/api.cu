@@ -421,13 +421,12 @@ static int launch_relayout(const void* src0, void* dst0, const ScaleLayout& L0, 
 }
 
 // D = epilogue(the slabs' sum, C); no slabs: k == 0.
-static int launch_reduce(bool is_mx, const EpilogueParams& epi, const uint32_t* ws, int slices, int64_t slab, int Mk,
-                         int Nk, int64_t ws_sr, int64_t ws_sc, int sms, cudaStream_t stream) {
+static int launch_reduce(bool is_mx, const EpilogueParams& epi, const uint32_t* ws, int slices, int Mk, int Nk, int sms,
+                         cudaStream_t stream) {
   const int threads = 256;
-  const int64_t total = static_cast<int64_t>(Mk) * Nk;
+  const int64_t tiles = static_cast<int64_t>((Mk + 31) / 32) * ((Nk + 7) / 8);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(
-      std::max<int64_t>(1, std::min<int64_t>((total + threads - 1) / threads, static_cast<int64_t>(sms) * 16))));
+  cfg.gridDim = dim3(static_cast<unsigned>(std::min<int64_t>(tiles, static_cast<int64_t>(sms) * 16)));
   cfg.blockDim = dim3(threads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -436,9 +435,9 @@ static int launch_reduce(bool is_mx, const EpilogueParams& epi, const uint32_t* 
   cfg.attrs = attr;
   cfg.numAttrs = env_switches().no_pdl || g_profile.load() ? 0 : 1;
   if (is_mx) {
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_epilogue_kernel<false>, epi, ws, slices, slab, Mk, Nk, ws_sr, ws_sc));
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_epilogue_kernel<false>, epi, ws, slices, Mk, Nk));
   } else {
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_epilogue_kernel<true>, epi, ws, slices, slab, Mk, Nk, ws_sr, ws_sc));
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_epilogue_kernel<true>, epi, ws, slices, Mk, Nk));
   }
   g_launches.fetch_add(1);
   CUDA_TRY(cudaGetLastError());
@@ -1047,7 +1046,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
 
   if (k == 0) {
     // D = epilogue(0, C): run_blocked.h:30-36.  Kernel view == caller view here.
-    if (int rc = launch_reduce(is_mx, epi, nullptr, 0, 0, m, n, c_rm ? n : 1, c_rm ? 1 : m, sms, stream)) return rc;
+    if (int rc = launch_reduce(is_mx, epi, nullptr, 0, m, n, sms, stream)) return rc;
   } else if (dp.use) {
     // ---- decode kernel: W = the caller's B on the MMA M side, X = the caller's A ---------------
     CUtensorMap tmW, tmX;
@@ -1274,18 +1273,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     }
     p.mode = ch.slices > 1 ? kModePartial : kModeEpilogue;
     p.epi = epi;
-    if (ch.slices > 1) {
-      p.ws = wsp + off_ws;
-      p.ws_slab = static_cast<int64_t>(Mk) * Nk;
-      // compact slab order follows D's contiguous direction in kernel view
-      if (epi.d_sr == 1) {
-        p.ws_sr = 1;
-        p.ws_sc = Mk;
-      } else {
-        p.ws_sr = Nk;
-        p.ws_sc = 1;
-      }
-    }
+    if (ch.slices > 1) p.ws = wsp + off_ws;
     if (is_mx) {
       p.sfa = sfa_dev;
       p.sfb = sfb_dev;
@@ -1461,9 +1449,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       g_profile_events.emplace_back(ev0, ev1);
     }
     if (ch.slices > 1) {
-      if (int rc = launch_reduce(is_mx, epi, static_cast<const uint32_t*>(p.ws), ch.slices, p.ws_slab, Mk, Nk, p.ws_sr,
-                                 p.ws_sc, sms, stream))
-        return rc;
+      if (int rc = launch_reduce(is_mx, epi, static_cast<const uint32_t*>(p.ws), ch.slices, Mk, Nk, sms, stream)) return rc;
     }
   }
 
@@ -1692,14 +1678,6 @@ CPUOPS_B200_API int cpuops_b200_gemm_i8_noalloc(const cpuops_b200_gemm_desc* d) 
   p.mode = kModePartial;
   p.epi = epi;
   p.ws = slabs;
-  p.ws_slab = static_cast<int64_t>(m) * n;
-  if (epi.d_sr == 1) {  // slab order follows D's contiguous direction
-    p.ws_sr = 1;
-    p.ws_sc = m;
-  } else {
-    p.ws_sr = n;
-    p.ws_sc = 1;
-  }
   p.error = error_word;
   p.wait_budget_us = g_wait_budget_us.load();
   const int per_stage = gemm_stage_bytes(BN);
@@ -1713,8 +1691,7 @@ CPUOPS_B200_API int cpuops_b200_gemm_i8_noalloc(const cpuops_b200_gemm_desc* d) 
                                                                             tmA, tmA /*unused: MX pair only*/, p);
   g_launches.fetch_add(1);
   CUDA_TRY(cudaGetLastError());
-  if (int rc = launch_reduce(false, epi, slabs, slices, p.ws_slab, m, n, p.ws_sr, p.ws_sc, nd->sm_count, stream))
-    return rc;
+  if (int rc = launch_reduce(false, epi, slabs, slices, m, n, nd->sm_count, stream)) return rc;
 
   int32_t device_error = 0;
   CUDA_TRY(cudaMemcpyAsync(&device_error, error_word, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));

@@ -172,16 +172,11 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, uint32_t (&r)[3
                                             uint32_t d_smem_row, int c_swz) {
   const int ncols = min(32, p.Nk - kcol0);
   if (p.mode == kModePartial) {
-    uint32_t* w = static_cast<uint32_t*>(p.ws) + (slice * p.ws_slab + krow * p.ws_sr + kcol0 * p.ws_sc);
-    if (p.ws_sc == 1 && ncols == 32 && aligned16(w)) {
+    // column by column: the warp's 32 rows are contiguous
+    uint32_t* w = static_cast<uint32_t*>(p.ws) + ((static_cast<int64_t>(slice) * p.Nk + kcol0) * p.Mk + krow);
 #pragma unroll
-      for (int i = 0; i < 32; i += 4)
-        *reinterpret_cast<uint4*>(w + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (i < ncols) w[i * p.ws_sc] = r[i];
-    }
+    for (int i = 0; i < 32; ++i, w += p.Mk)
+      if (i < ncols) *w = r[i];
     return;
   }
   const EpilogueParams& e = p.epi;
@@ -787,7 +782,7 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
       const uint32_t nb = static_cast<uint32_t>(p.ring_bufs);
       asm volatile("griddepcontrol.wait;" ::: "memory");  // before C is read, D or a slab written
       warm_epilogue_params(p.epi);  // constant-cache misses now, not after the first accumulator
-      asm volatile("" ::"r"(p.Mk ^ p.Nk ^ p.mode), "l"(p.ws), "l"(p.ws_slab ^ p.ws_sr ^ p.ws_sc));
+      asm volatile("" ::"r"(p.Mk ^ p.Nk ^ p.mode), "l"(p.ws));
       const uint32_t my_c = c_base + static_cast<uint32_t>(ew) * nb * 4096u;
       uint32_t cq = 0;        // chunks consumed so far by this warp
       uint32_t cq_b = 0, cq_ph = 0;  // its buffer and that buffer's barrier parity

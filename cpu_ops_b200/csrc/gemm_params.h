@@ -73,9 +73,7 @@ struct GemmParams {
   uint32_t idesc;           // instruction descriptor without scale-factor ids
   int32_t mode;             // kModeEpilogue | kModePartial
   EpilogueParams epi;
-  // split-k slabs: element (s, krow, kcol) at ws[s*ws_slab + krow*ws_sr + kcol*ws_sc]
-  void* ws;
-  int64_t ws_slab, ws_sr, ws_sc;
+  void* ws;                 // split-k slabs: element (s, krow, kcol) at ws[(s * Nk + kcol) * Mk + krow]
   // MX: re-laid-out scale factors, one contiguous chunk per (tile, stage)
   const uint8_t* sfa;
   const uint8_t* sfb;
