@@ -799,12 +799,15 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     if (d->split_k_slices > 1) {
       ch.slices = std::min(d->split_k_slices, k_blocks);
     } else if (d->split_k_slices == 0 && tiles < 2 * sms && k_blocks >= 8) {
-      // Few tiles and a deep k: cut k so that the work items fill the SMs.  Time
-      // estimate (microseconds): waves x k-blocks per slice x per-block time, plus
-      // the slab write + read and one more launch when split.
-      const double hbm_bytes_per_us = 6.0e6, per_sm = hbm_bytes_per_us / sms;
-      const double block_us = std::max(gemm_stage_bytes(ch.BN) / per_sm,
-                                       4.0 * std::max(ch.BN / 2.0, (128.0 + ch.BN) / 4.0) / 1500.0);
+      // Few tiles and a deep k: cut k so that the work items fill the SMs.  Estimate in
+      // microseconds, fitted to calls on 64 x 128 .. 1024 x 1024 outputs with k = 4096 .. 32768 in 1
+      // to 24 slices: waves x k-blocks per slice x 0.13 (BN 128; 8-bit MX 0.21), and when split
+      // the second launch and the slabs, 1 + 9 per million outputs + 0.17 per slice (8-bit
+      // MX 2 more: it has its scales re-laid-out then).  Chosen by an estimate that charged every
+      // CTA an SM's share of HBM, before / now: u8 x s8 192 x 320 x 16384 (22 / 8 slices) 12.4 / 9.7 us,
+      // 640 x 1024 x 8192 (3 / 1) 17.5 / 15.7, 1024 x 1024 x 8192 (2 / 1) 23.0 / 18.4.
+      const double block_us = (kind == kKindMxf8 ? 0.21 : 0.13) * std::max(1.0, (128.0 + ch.BN) / 256.0);
+      const double split_us = 1.0 + 9e-6 * Mk * static_cast<double>(Nk) + (kind == kKindMxf8 ? 2.0 : 0.0);
       double best = 1e300;
       // unsplit, a ragged last tile column is computed narrower and dealt out evenly:
       // rounds in units of a wide tile (feed-bound cost ~ 128 + width rows per k-block)
@@ -819,7 +822,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
         const int64_t waves = (tiles * s + sms - 1) / sms;
         const int per_slice = (k_blocks + s - 1) / s;
         double t_us = (s == 1 ? rounds1 : static_cast<double>(waves)) * per_slice * block_us;
-        if (s > 1) t_us += 2.0 * s * Mk * static_cast<double>(Nk) * 4.0 / hbm_bytes_per_us + 3.0;
+        if (s > 1) t_us += split_us + 0.17 * s;
         if (t_us < best * 0.97) {
           best = t_us;
           ch.slices = s;
