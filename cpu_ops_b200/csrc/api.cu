@@ -794,41 +794,55 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       set_error("tile_n %d is not usable here", ch.BN);
       return CPUOPS_B200_STATUS_INVALID_ARGUMENTS;
     }
-    ch.nacc = (is_mx && ch.BN > 224) ? 1 : 2;
-    const int64_t tiles = static_cast<int64_t>((Mk + 127) / 128) * ((Nk + ch.BN - 1) / ch.BN);
-    if (d->split_k_slices > 1) {
-      ch.slices = std::min(d->split_k_slices, k_blocks);
-    } else if (d->split_k_slices == 0 && tiles < 2 * sms && k_blocks >= 8) {
-      // Few tiles and a deep k: cut k so that the work items fill the SMs.  Estimate in
-      // microseconds, fitted to calls on 64 x 128 .. 1024 x 1024 outputs with k = 4096 .. 32768 in 1
-      // to 24 slices: waves x k-blocks per slice x 0.13 (BN 128; 8-bit MX 0.21), and when split
-      // the second launch and the slabs, 1 + 9 per million outputs + 0.17 per slice (8-bit
-      // MX 2 more: it has its scales re-laid-out then).  Chosen by an estimate that charged every
-      // CTA an SM's share of HBM, before / now: u8 x s8 192 x 320 x 16384 (22 / 8 slices) 12.4 / 9.7 us,
-      // 640 x 1024 x 8192 (3 / 1) 17.5 / 15.7, 1024 x 1024 x 8192 (2 / 1) 23.0 / 18.4.
-      const double block_us = (kind == kKindMxf8 ? 0.21 : 0.13) * std::max(1.0, (128.0 + ch.BN) / 256.0);
+    // Few tiles and a deep k: cut k so that the work items fill the SMs.  Estimate in
+    // microseconds, fitted to calls on 64 x 128 .. 1024 x 1024 outputs with k = 4096 .. 32768 in 1
+    // to 24 slices: waves x k-blocks per slice x 0.13 (BN 128; 8-bit MX 0.21), and when split
+    // the second launch and the slabs, 1 + 9 per million outputs + 0.17 per slice (8-bit
+    // MX 2 more: it has its scales re-laid-out then).  Chosen by an estimate that charged every
+    // CTA an SM's share of HBM, before / now: u8 x s8 192 x 320 x 16384 (22 / 8 slices) 12.4 / 9.7 us,
+    // 640 x 1024 x 8192 (3 / 1) 17.5 / 15.7, 1024 x 1024 x 8192 (2 / 1) 23.0 / 18.4.
+    auto estimate = [&](int BN, int* slices) {
+      const int n_tiles = (Nk + BN - 1) / BN, m_tiles = (Mk + 127) / 128, last = last_tile_width(Nk, BN);
+      const int64_t tiles = static_cast<int64_t>(m_tiles) * n_tiles;
+      const double block_us = (kind == kKindMxf8 ? 0.21 : 0.13) * (128.0 + BN) / 256.0;
       const double split_us = 1.0 + 9e-6 * Mk * static_cast<double>(Nk) + (kind == kKindMxf8 ? 2.0 : 0.0);
       double best = 1e300;
       // unsplit, a ragged last tile column is computed narrower and dealt out evenly:
       // rounds in units of a wide tile (feed-bound cost ~ 128 + width rows per k-block)
       double rounds1 = static_cast<double>((tiles + sms - 1) / sms);
-      {
-        const int n_tiles = (Nk + ch.BN - 1) / ch.BN, m_tiles = (Mk + 127) / 128, last = last_tile_width(Nk, ch.BN);
-        if (!bk_role_mn && n_tiles >= 2 && last < ch.BN && !env_switches().no_narrow)
-          rounds1 = busiest_worker(m_tiles * (n_tiles - 1), m_tiles, sms, 1.0,
-                                   (128.0 + last) / (128.0 + ch.BN));
-      }
-      for (int s = 1; s <= std::min(32, k_blocks / 2); ++s) {
+      if (!bk_role_mn && n_tiles >= 2 && last < BN && !env_switches().no_narrow)
+        rounds1 = busiest_worker(m_tiles * (n_tiles - 1), m_tiles, sms, 1.0, (128.0 + last) / (128.0 + BN));
+      const bool may_split = d->split_k_slices == 0 && tiles < 2 * sms && k_blocks >= 8;
+      for (int s = 1; s <= (may_split ? std::min(32, k_blocks / 2) : 1); ++s) {
         const int64_t waves = (tiles * s + sms - 1) / sms;
         const int per_slice = (k_blocks + s - 1) / s;
         double t_us = (s == 1 ? rounds1 : static_cast<double>(waves)) * per_slice * block_us;
         if (s > 1) t_us += split_us + 0.17 * s;
         if (t_us < best * 0.97) {
           best = t_us;
-          ch.slices = s;
+          *slices = s;
+        }
+      }
+      return best;
+    };
+    if (d->split_k_slices > 1) {
+      ch.slices = std::min(d->split_k_slices, k_blocks);
+    } else {
+      const double us = estimate(ch.BN, &ch.slices);
+      // 64-wide tiles where even those run all at once: twice the CTAs, each with half the epilogue
+      // (about 0.016 us per column).  BN 128 / 64: u8 x s8 512^3 6.2 / 5.1 us, 1024^3 6.7 / 5.8, 128 x
+      // 4096 x 4096 10.7 / 8.9, 300 x 1000 x 2000 11.0 / 8.8; e4m3 512 x 2048 x 1024 + bias + SiLU 11.2 /
+      // 9.3, 128 x 4096 x 4096 14.3 / 12.2; e2m1 512 x 2048 x 1024 7.6 / 7.0.
+      const int64_t narrow_tiles = static_cast<int64_t>((Mk + 127) / 128) * ((Nk + 63) / 64);
+      if (d->tile_n == 0 && !bk_role_mn && ch.BN > 64 && narrow_tiles <= sms && !(d->flags & CPUOPS_B200_FLAG_PAIR_ON)) {
+        int slices = 1;
+        if (estimate(64, &slices) + 0.016 * 64 < us + 0.016 * ch.BN) {
+          ch.BN = 64;
+          ch.slices = slices;
         }
       }
     }
+    ch.nacc = (is_mx && ch.BN > 224) ? 1 : 2;
   }
 
   // ---- one CTA per tile, or a pair of CTAs per 256-row tile ---------------------------------
@@ -1321,12 +1335,12 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     p.ring_bufs = (p.c_ring || p.d_ring) ? 2 : 0;
     if (p.ring_bufs && env_switches().ring == 3) p.ring_bufs = 3;
     // Eight epilogue warps (two per tensor-memory lane quarter) when no CTA gets a second
-    // tile to hide its epilogue behind and the tile is wide enough to share out; otherwise
+    // tile to hide its epilogue behind and the tile has two chunks to share out; otherwise
     // four, which leave more shared memory to the k pipeline.
     int epi_warps = 4;
     {
       const int64_t items = static_cast<int64_t>(p.m_tiles) * p.n_tiles * p.slices;
-      if (items * (ch.pair ? 2 : 1) <= sms && ch.BN >= 128) epi_warps = 8;
+      if (items * (ch.pair ? 2 : 1) <= sms && ch.BN >= 64) epi_warps = 8;
       // ... or when k is so short that a tile's k loop (about 600 cycles per k-block) ends
       // well before four warps have drained the previous tile (about 1500 cycles per
       // 32-column chunk each): measured +10-15 % at K = 1024, nothing at K = 2048

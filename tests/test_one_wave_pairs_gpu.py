@@ -26,3 +26,21 @@ def test_pairs_in_one_wave(gpu, m, n, k, beta, pair):
         assert _capi.last_plan().pair == pair
     # |sums| < 2^53: exact in f64
     assert torch.equal(D, (A.double() @ B.double().T).to(torch.int32) + beta * C)
+
+
+@pytest.mark.parametrize("m,n,k,tile_n", [(512, 512, 512, 64), (1000, 900, 300, 64), (129, 65, 128, 64), (1024, 1216, 512, 128),
+                                          (128, 9472, 256, 64), (100, 200, 1500, 64), (60, 70, 333, 64)])
+def test_narrow_tiles_in_one_wave(gpu, m, n, k, tile_n):
+    """64-wide tiles while all of them run at once (1024 x 1216: 152 tiles on 148 SMs do not)."""
+    k = (k + 15) // 16 * 16
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    A = torch.randint(0, 256, (m, k), dtype=torch.uint8, device="cuda", generator=g)
+    B = torch.randint(-128, 128, (n, k), dtype=torch.int8, device="cuda", generator=g)
+    C = torch.randint(-1000, 1000, (m, n), dtype=torch.int32, device="cuda", generator=g)
+    D = torch.full((m, n), 77, dtype=torch.int32, device="cuda")
+    op = c.GemmU8S8S32(c.RowMajor, c.ColumnMajor, c.RowMajor)
+    st = op(op.Arguments(c.GemmCoord(m, n, k), c.TensorRef(A, k), c.TensorRef(B, k), c.TensorRef(C, n),
+                         c.TensorRef(D, n), c.LinearCombination(1, 1), 1))
+    assert st == c.Status.kSuccess, _capi.last_error()
+    assert (_capi.last_plan().tile_n <= 64) == (tile_n == 64)
+    assert torch.equal(D, (A.double() @ B.double().T).to(torch.int32) + C)
