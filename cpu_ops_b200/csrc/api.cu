@@ -773,6 +773,14 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   B.inner_bytes = b_kmajor ? row_bytes(fp4_b, k) : n;
   B.pitch = fp4_b ? d->ldb / 2 : d->ldb;
 
+  // Whether every row of both scale arrays starts at a multiple of `to` bytes.
+  auto scale_rows_aligned = [&](int to) {
+    auto aligned = [&](const void* ptr, bool on_device, int ld, int rows) {
+      return (!on_device || reinterpret_cast<uintptr_t>(ptr) % to == 0) && (rows <= 1 || ld % to == 0);
+    };
+    return aligned(d->a_scales, sa_dev, d->ld_scales_a, m) && aligned(d->b_scales, sb_dev, d->ld_scales_b, n);
+  };
+
   // ---- configuration -----------------------------------------------------------------
   Choice ch;
   const bool fp4_pair = fp4_a && fp4_b;
@@ -797,15 +805,15 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
     // Few tiles and a deep k: cut k so that the work items fill the SMs.  Estimate in
     // microseconds, fitted to calls on 64 x 128 .. 1024 x 1024 outputs with k = 4096 .. 32768 in 1
     // to 24 slices: waves x k-blocks per slice x 0.13 (BN 128; 8-bit MX 0.21), and when split
-    // the second launch and the slabs, 1 + 9 per million outputs + 0.17 per slice (8-bit
-    // MX 2 more: it has its scales re-laid-out then).  Chosen by an estimate that charged every
+    // the second launch and the slabs, 1 + 9 per million outputs + 0.17 per slice (8-bit MX
+    // 2 more where its scales have to be re-laid-out).  Chosen by an estimate that charged every
     // CTA an SM's share of HBM, before / now: u8 x s8 192 x 320 x 16384 (22 / 8 slices) 12.4 / 9.7 us,
     // 640 x 1024 x 8192 (3 / 1) 17.5 / 15.7, 1024 x 1024 x 8192 (2 / 1) 23.0 / 18.4.
     auto estimate = [&](int BN, int* slices) {
       const int n_tiles = (Nk + BN - 1) / BN, m_tiles = (Mk + 127) / 128, last = last_tile_width(Nk, BN);
       const int64_t tiles = static_cast<int64_t>(m_tiles) * n_tiles;
       const double block_us = (kind == kKindMxf8 ? 0.21 : 0.13) * (128.0 + BN) / 256.0;
-      const double split_us = 1.0 + 9e-6 * Mk * static_cast<double>(Nk) + (kind == kKindMxf8 ? 2.0 : 0.0);
+      const double split_us = 1.0 + 9e-6 * Mk * static_cast<double>(Nk) + (kind == kKindMxf8 && !scale_rows_aligned(4) ? 2.0 : 0.0);
       double best = 1e300;
       // unsplit, a ragged last tile column is computed narrower and dealt out evenly:
       // rounds in units of a wide tile (feed-bound cost ~ 128 + width rows per k-block)
@@ -866,12 +874,6 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   // (one launch, raw scales, every SM streaming an equal share of the weights).  It fetches the
   // scale rows 16 bytes at a time, which wants 16-byte aligned bases and leading dimensions; a
   // forced tile width or slice count keeps the general kernel, whose plan those describe.
-  auto scale_rows_aligned = [&](int to) {
-    auto aligned = [&](const void* ptr, bool on_device, int ld, int rows) {
-      return (!on_device || reinterpret_cast<uintptr_t>(ptr) % to == 0) && (rows <= 1 || ld % to == 0);
-    };
-    return aligned(d->a_scales, sa_dev, d->ld_scales_a, m) && aligned(d->b_scales, sb_dev, d->ld_scales_b, n);
-  };
   DecodePlan dp;
   if (k > 0 && is_mx && !mixed && ch.swap && m <= 64 && d->tile_n == 0 && d->split_k_slices <= 1 &&
       !(d->flags & (CPUOPS_B200_FLAG_PAIR_ON | CPUOPS_B200_FLAG_PAIR_OFF)) && !env_switches().no_decode) {
@@ -883,16 +885,17 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
   // one CTA per tile.  e4m3 and e5m2 gain while the launch is short; over many k-blocks the
   // longer way to a full stage costs more than the re-layout: e4m3 re-laid-out / raw, k-blocks
   // that a CTA runs through: 4500 x 4500 x 640 (26) 37.4 / 34.0 us, 2048 x 3072 x 2048 (28) 23.7 / 22.2,
-  // 8192 x 4096 x 512 (33) 44.8 / 46, 2304 x 2304 x 4096 (58) 29.2 / 32.1, and with split k 128 x 8192 x
-  // 4096 27.5 / 28.7.  One tile per CTA hides more: 1100 x 4096 x 4096 (32) 31.1 / 25.4, 256 x 8192 x
-  // 8192 (64) 36.6 / 31.3.  A k-block's words must be aligned in every row: four bytes, e2m1 eight.
+  // 8192 x 4096 x 512 (33) 44.8 / 46, 2304 x 2304 x 4096 (58) 29.2 / 32.1.  One work item per CTA hides
+  // more: 1100 x 4096 x 4096 (32) 31.1 / 25.4, 256 x 8192 x 8192 (64) 36.6 / 31.3, in eight slices 100 x
+  // 500 x 8192 12.1 / 9.2, 192 x 320 x 16384 14.3 / 12.0.  A k-block's words must be aligned in every row: four bytes, e2m1 eight.
   bool raw_scales = false;
   if (is_mx && k > 0 && !mixed && !dp.use && !ch.pair && scale_rows_aligned(fp4_pair ? 8 : 4)) {
     const int Mk = ch.swap ? n : m, Nk = ch.swap ? m : n;
     const int64_t items = static_cast<int64_t>((Mk + 127) / 128) * ((Nk + ch.BN - 1) / ch.BN);
-    raw_scales = fp4_pair || (ch.slices == 1 && (items <= sms || items * k_blocks <= 32 * static_cast<int64_t>(sms)));
+    raw_scales = fp4_pair || items * ch.slices <= sms ||
+                 (ch.slices == 1 && items * k_blocks <= 32 * static_cast<int64_t>(sms));
+    if (env_switches().raw >= 0) raw_scales = env_switches().raw != 0;
   }
-  if (env_switches().raw >= 0) raw_scales = raw_scales && env_switches().raw != 0;
   if (raw_scales && sb_dev) {
     std::lock_guard<std::mutex> registry_lock(g_registry_mu);
     if (find_prepared(st.device, d->b_scales, n, k, d->ld_scales_b)) raw_scales = false;
