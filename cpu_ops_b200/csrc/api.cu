@@ -58,6 +58,7 @@ struct Choice {
   int nacc = 2;
   int slices = 1;
   int stages = 4;
+  int piece_kb = 0;   // 8-bit MX: k-blocks summed in one accumulator (k_blocks: all)
 };
 
 int pick_bn_for_small(int nk) {
@@ -547,7 +548,7 @@ CPUOPS_B200_API int cpuops_b200_profile_collect(double* total_ms, int32_t* launc
 // The whole call.  depth 0: a caller's descriptor; takes the device's lock.  depth 1: one
 // row panel of a host-operand call, issued by depth 0 on one of the panel streams
 // (asynchronous, with host pointers allowed: the parent synchronises and holds the lock).
-static int gemm_body(const cpuops_b200_gemm_desc* d, int depth);
+static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece_kb = 0);
 
 extern "C" {
 
@@ -621,7 +622,7 @@ static int run_host_row_panels(const cpuops_b200_gemm_desc* d, DeviceState& st, 
     for (int t = 0; t < pd.n_ops; ++t)
       if (pd.ops[t].opcode == CPUOPS_B200_OP_SCALE_PER_ROW)
         pd.ops[t].ptr = static_cast<const uint8_t*>(d->ops[t].ptr) + static_cast<int64_t>(row0) * 4;
-    if (int rc = gemm_body(&pd, 1)) {
+    if (int rc = gemm_body(&pd, 1, ch.piece_kb)) {
       for (int q = 0; q < DeviceState::kPanelStreams; ++q) cudaStreamSynchronize(st.panel_stream[q]);
       return rc;
     }
@@ -704,7 +705,7 @@ static int validate_descriptor(const cpuops_b200_gemm_desc* d, bool* finished) {
   return CPUOPS_B200_STATUS_SUCCESS;
 }
 
-static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
+static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece_kb) {
   {
     bool finished = false;
     const int rc = validate_descriptor(d, &finished);
@@ -833,20 +834,54 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
       }
       return best;
     };
+    // 8-bit MX: how many parts k would be cut into if every CTA had only an SM's share of HBM
+    // bandwidth to feed it.  The tensor cores lose low bits along a running sum, so this is
+    // also how often a sum starts afresh: a launch with fewer slices than this keeps the
+    // precision by summing in pieces (piece_kb), and one that cannot (BN > 64) keeps the slices.
+    auto precision_parts = [&](int BN) {
+      const int64_t tiles = static_cast<int64_t>((Mk + 127) / 128) * ((Nk + BN - 1) / BN);
+      int parts = 1;
+      if (tiles >= 2 * sms || k_blocks < 8) return parts;
+      const double hbm_bytes_per_us = 6.0e6, block_us = gemm_stage_bytes(BN) * sms / hbm_bytes_per_us;
+      const int n_tiles = (Nk + BN - 1) / BN, m_tiles = (Mk + 127) / 128, last = last_tile_width(Nk, BN);
+      double best = 1e300, rounds1 = static_cast<double>((tiles + sms - 1) / sms);
+      if (n_tiles >= 2 && last < BN)
+        rounds1 = busiest_worker(m_tiles * (n_tiles - 1), m_tiles, sms, 1.0, (128.0 + last) / (128.0 + BN));
+      for (int s = 1; s <= std::min(32, k_blocks / 2); ++s) {
+        double t_us = (s == 1 ? rounds1 : static_cast<double>((tiles * s + sms - 1) / sms)) * ((k_blocks + s - 1) / s) * block_us;
+        if (s > 1) t_us += 2.0 * s * Mk * static_cast<double>(Nk) * 4.0 / hbm_bytes_per_us + 3.0;
+        if (t_us < best * 0.97) {
+          best = t_us;
+          parts = s;
+        }
+      }
+      return parts;
+    };
+    ch.piece_kb = parent_piece_kb > 0 ? parent_piece_kb : k_blocks;
     if (d->split_k_slices > 1) {
       ch.slices = std::min(d->split_k_slices, k_blocks);
     } else {
+      const int parts = kind == kKindMxf8 && d->split_k_slices == 0 ? precision_parts(ch.BN) : 1;
+      // a caller that asks for one of the two forms gets the same tile, slices and bits in either
+      const bool form_given = (d->flags & (CPUOPS_B200_FLAG_PAIR_ON | CPUOPS_B200_FLAG_PAIR_OFF)) != 0;
       const double us = estimate(ch.BN, &ch.slices);
       // 64-wide tiles where even those run all at once: twice the CTAs, each with half the epilogue
       // (about 0.016 us per column).  BN 128 / 64: u8 x s8 512^3 6.2 / 5.1 us, 1024^3 6.7 / 5.8, 128 x
       // 4096 x 4096 10.7 / 8.9, 300 x 1000 x 2000 11.0 / 8.8; e4m3 512 x 2048 x 1024 + bias + SiLU 11.2 /
-      // 9.3, 128 x 4096 x 4096 14.3 / 12.2; e2m1 512 x 2048 x 1024 7.6 / 7.0.
+      // 9.6, 128 x 4096 x 4096 14.3 / 12.2; e2m1 512 x 2048 x 1024 7.6 / 7.0.
       const int64_t narrow_tiles = static_cast<int64_t>((Mk + 127) / 128) * ((Nk + 63) / 64);
-      if (d->tile_n == 0 && !bk_role_mn && ch.BN > 64 && narrow_tiles <= sms && !(d->flags & CPUOPS_B200_FLAG_PAIR_ON)) {
+      if (d->tile_n == 0 && !bk_role_mn && ch.BN > 64 && narrow_tiles <= sms && !form_given) {
         int slices = 1;
-        if (estimate(64, &slices) + 0.016 * 64 < us + 0.016 * ch.BN) {
+        if (estimate(64, &slices) + 0.016 * 64 < us + 0.016 * ch.BN || parts > 1) {
           ch.BN = 64;
           ch.slices = slices;
+        }
+      }
+      if (parts > 1) {
+        if (ch.BN <= 64 && !form_given) {  // (pairs sum k in one piece)
+          ch.piece_kb = std::max(1, k_blocks / parts);
+        } else {
+          ch.slices = parts;
         }
       }
     }
@@ -1361,6 +1396,14 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth) {
             p.mode == kModeEpilogue && k_blocks <= 32 && ch.BN >= 128)
           epi_warps = 8;
       if (env_switches().epi_warps == 8 || env_switches().epi_warps == 4) epi_warps = env_switches().epi_warps;
+    }
+    // 8-bit MX tiles with at most one 32-column chunk per epilogue warp may be summed in pieces,
+    // added in f32 by those warps behind the MMAs (kPieces in gemm_kernel.cuh; wider tiles have
+    // more accumulators than a warp has registers for).
+    p.piece_kb = k_blocks;
+    if (kind == kKindMxf8 && !ch.pair && ch.BN <= 64 && ch.piece_kb < k_blocks) {
+      epi_warps = 8;
+      p.piece_kb = ch.piece_kb;
     }
     p.error = st.error_dev;
     p.wait_budget_us = g_wait_budget_us.load();

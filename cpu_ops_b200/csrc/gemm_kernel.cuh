@@ -369,6 +369,11 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
   constexpr bool kMx = !kInt;
   static_assert(!kRaw || (kMx && !kPair), "raw scales: MX operands, one CTA per tile");
   constexpr int kCtas = kPair ? 2 : 1;
+  // 8-bit MX, one CTA per tile: the accumulator may be taken down every p.piece_kb k-blocks and
+  // the pieces added by the epilogue warps.  The tensor cores drop the low bits of a running
+  // sum: against float64, results are off by 6e-10 per element of k (2.4e-6 at k = 4096), and
+  // by 2e-7 at any k in pieces of 256 elements.
+  constexpr bool kPieces = KIND == kKindMxf8 && !kPair;
   // Programmatic dependent launch: the next kernel in the stream may become resident as
   // this one's CTAs retire; in return every role of this kernel that touches global memory
   // first waits for the kernel before it (griddepcontrol.wait), so stream order holds.
@@ -659,17 +664,30 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
       uint32_t a_lo = a_lo0, b_lo = b_lo0, full_addr = full0, empty_addr = empty0, sf_lo = sf_lo0;
       for (int t = work0; t < total_tiles && ok; t += work_step) {
         const TileCoord tc = decode_tile(p, t, work_step);
-        long long tw0 = dbg ? clock64() : 0;
-        if (!__all_sync(kAll, mbar_wait_bounded(acc_empty_bar(buf), acc_ph ^ 1u, abort_flag, budget_ns))) {
-          if (el) record_error(p, abort_flag, kErrMmaWaitAcc);
-          break;
-        }
-        if (dbg) dbg_wait_acc += clock64() - tw0;
-        tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * p.BN);
         if (p.narrow_last) set_idesc_width(tc.bn);
-        uint32_t accumulate = 0;
+        uint32_t accumulate = 0, d_tmem = 0;
+        int piece_end = 0;  // the k-block at which the accumulator changes
         for (int i = 0; i < tc.nkb; ++i) {
+          long long tw0 = dbg ? clock64() : 0;
+          if (i == piece_end) {
+            if (kPieces && i > 0) {
+              tc_commit_both<kPair>(acc_full_bar(buf), el);
+              if (++buf == nacc) {
+                buf = 0;
+                acc_ph ^= 1u;
+              }
+            }
+            if (!__all_sync(kAll, mbar_wait_bounded(acc_empty_bar(buf), acc_ph ^ 1u, abort_flag, budget_ns))) {
+              if (el) record_error(p, abort_flag, kErrMmaWaitAcc);
+              ok = false;
+              break;
+            }
+            if (dbg) dbg_wait_acc += clock64() - tw0;
+            tc_fence_after_sync();
+            d_tmem = tmem_base + static_cast<uint32_t>(buf * p.BN);
+            accumulate = 0;
+            piece_end = kPieces ? min(i + p.piece_kb, tc.nkb) : tc.nkb;
+          }
           tw0 = dbg ? clock64() : 0;
           if (!peek && !__all_sync(kAll, mbar_wait_bounded(full_addr, ph, abort_flag, budget_ns))) {
             if (el) record_error(p, abort_flag, kErrMmaWaitFull);
@@ -805,8 +823,6 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
       };
       for (int t = work0; t < total_tiles && alive; t += work_step, ++it) {
         const TileCoord tc = decode_tile(p, t, work_step);
-        const int buf = it % nacc;
-        const uint32_t acc_ph = static_cast<uint32_t>(it / nacc) & 1u;
         const int row0 = (tc.m_tile * kCtas + static_cast<int>(cta_rank)) * kTileM + q * 32;
         const int krow = row0 + lane;
         const int n0 = tc.n_tile * p.BN;
@@ -821,6 +837,42 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
             if (!kTmaOnly && !c_tma) cp_async_commit();
           }
         }
+        // All pieces of the tile but the last (at most one chunk per warp then).
+        [[maybe_unused]] uint32_t sum[32];
+        [[maybe_unused]] bool summed = false;
+        if constexpr (kPieces) {
+          for (int left = tc.nkb; left > p.piece_kb; left -= p.piece_kb, ++it) {
+            const int pb = it % nacc;
+            const bool got = mbar_wait_bounded(acc_full_bar(pb), static_cast<uint32_t>(it / nacc) & 1u, abort_flag, budget_ns);
+            if (!__all_sync(0xffffffffu, got)) {
+              alive = false;
+              break;
+            }
+            tc_fence_after_sync();
+            if (c0 < nchunks) {
+              const uint32_t from = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(pb * p.BN + c0 * 32);
+#pragma unroll
+              for (int h = 0; h < 32; h += 16) {  // (16 at a time: the raw kernels have 128 registers)
+                uint32_t v[16];
+                tmem_ld_32x16(from + static_cast<uint32_t>(h), v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                  sum[h + i] = summed ? __float_as_uint(__fadd_rn(__uint_as_float(sum[h + i]), __uint_as_float(v[i]))) : v[i];
+              }
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty_bar(pb));
+            summed = true;
+          }
+          if (!alive) {
+            if (lane == 0) record_error(p, abort_flag, kErrEpilogueWait);
+            break;
+          }
+        }
+        const int buf = it % nacc;
+        const uint32_t acc_ph = static_cast<uint32_t>(it / nacc) & 1u;
         const long long te0 = edbg ? clock64() : 0;
         const bool ready = mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
         if (!__all_sync(0xffffffffu, ready)) {
@@ -847,6 +899,15 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
           uint32_t r[32];
           tmem_ld_32x32(taddr + static_cast<uint32_t>(c * 32), r);
           tmem_ld_wait();
+          if constexpr (kPieces) {
+            if (summed) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__fadd_rn(__uint_as_float(sum[i]), __uint_as_float(r[i])));
+            }
+            summed = false;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sum[i] = 0u;  // (ends its life here: no registers behind this line)
+          }
           if (c + cstep >= nchunks) {
             // the accumulator is in registers: hand the buffer back to the MMA warp
             tc_fence_before_sync();
