@@ -665,96 +665,88 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
       for (int t = work0; t < total_tiles && ok; t += work_step) {
         const TileCoord tc = decode_tile(p, t, work_step);
         if (p.narrow_last) set_idesc_width(tc.bn);
-        uint32_t accumulate = 0, d_tmem = 0;
-        int piece_end = 0;  // the k-block at which the accumulator changes
-        for (int i = 0; i < tc.nkb; ++i) {
+        int i = 0;
+        do {  // one piece of k (kPieces; otherwise all of it: the k loop below pays nothing for this)
           long long tw0 = dbg ? clock64() : 0;
-          if (i == piece_end) {
-            if (kPieces && i > 0) {
-              tc_commit_both<kPair>(acc_full_bar(buf), el);
-              if (++buf == nacc) {
-                buf = 0;
-                acc_ph ^= 1u;
-              }
-            }
-            if (!__all_sync(kAll, mbar_wait_bounded(acc_empty_bar(buf), acc_ph ^ 1u, abort_flag, budget_ns))) {
-              if (el) record_error(p, abort_flag, kErrMmaWaitAcc);
-              ok = false;
-              break;
-            }
-            if (dbg) dbg_wait_acc += clock64() - tw0;
-            tc_fence_after_sync();
-            d_tmem = tmem_base + static_cast<uint32_t>(buf * p.BN);
-            accumulate = 0;
-            piece_end = kPieces ? min(i + p.piece_kb, tc.nkb) : tc.nkb;
-          }
-          tw0 = dbg ? clock64() : 0;
-          if (!peek && !__all_sync(kAll, mbar_wait_bounded(full_addr, ph, abort_flag, budget_ns))) {
-            if (el) record_error(p, abort_flag, kErrMmaWaitFull);
+          if (!__all_sync(kAll, mbar_wait_bounded(acc_empty_bar(buf), acc_ph ^ 1u, abort_flag, budget_ns))) {
+            if (el) record_error(p, abort_flag, kErrMmaWaitAcc);
             ok = false;
             break;
           }
-          if (dbg) dbg_wait_full += clock64() - tw0;
-          // probe the next ring slot now; the answer (a shared-memory round trip of about
-          // 100 cycles) is only read after this k-block's MMAs have been issued
-          const uint32_t nfull = (s + 1 == stages) ? full0 : full_addr + 8;
-          const uint32_t nph = (s + 1 == stages) ? (ph ^ 1u) : ph;
-          const uint32_t probe = mbar_test_wait(nfull, nph);
-          const uint32_t sfb_t = sfa_t + 4u * sfa_atoms;
+          if (dbg) dbg_wait_acc += clock64() - tw0;
           tc_fence_after_sync();
-          if constexpr (kMx) {
-            // this k-block's scale atoms: shared -> the slot's tensor-memory columns
-            uint32_t src = sf_lo, dst = sfa_t;
-            for (uint32_t a = 0; a < sf_atoms; ++a, src += 32, dst += 4)
-              tmem_cp_atom_g<kPair>(dst, src, sf_hi, el);
-          }
-          if constexpr (KIND == kKindI8) {
-            mma_i8_g<kPair>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, accumulate, el);
-            mma_i8_g<kPair>(d_tmem, a_lo + a_k, a_hi, b_lo + b_k, b_hi, idesc, 1u, el);
-            mma_i8_g<kPair>(d_tmem, a_lo + 2 * a_k, a_hi, b_lo + 2 * b_k, b_hi, idesc, 1u, el);
-            mma_i8_g<kPair>(d_tmem, a_lo + 3 * a_k, a_hi, b_lo + 3 * b_k, b_hi, idesc, 1u, el);
-          } else if constexpr (KIND == kKindMxf8) {
-            mma_mxf8f6f4_g<kPair>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, sfa_t, sfb_t, accumulate, el);
-            mma_mxf8f6f4_g<kPair>(d_tmem, a_lo + 2, a_hi, b_lo + 2, b_hi, id1, sfa_t, sfb_t, 1u, el);
-            mma_mxf8f6f4_g<kPair>(d_tmem, a_lo + 4, a_hi, b_lo + 4, b_hi, id2, sfa_t, sfb_t, 1u, el);
-            mma_mxf8f6f4_g<kPair>(d_tmem, a_lo + 6, a_hi, b_lo + 6, b_hi, id3, sfa_t, sfb_t, 1u, el);
-          } else {
-            mma_mxf4_g<kPair>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, sfa_t, sfb_t, accumulate, el);
-            mma_mxf4_g<kPair>(d_tmem, a_lo + 2, a_hi, b_lo + 2, b_hi, id1, sfa_t, sfb_t, 1u, el);
-            mma_mxf4_g<kPair>(d_tmem, a_lo + 4, a_hi, b_lo + 4, b_hi, id2, sfa_t + sfa_half, sfb_t + sfb_half, 1u, el);
-            mma_mxf4_g<kPair>(d_tmem, a_lo + 6, a_hi, b_lo + 6, b_hi, id3, sfa_t + sfa_half, sfb_t + sfb_half, 1u, el);
-          }
-          accumulate = 1u;
-          tc_commit_both<kPair>(empty_addr, el);  // frees the stage (in both CTAs) once these MMAs have read it
-          peek = __all_sync(kAll, probe != 0) ? 1u : 0u;
-          if constexpr (kMx) {
-            sfa_t += sf_cols;
-            if (++sf_q == sf_slots) {
-              sf_q = 0;
-              sfa_t = sf_t0;
+          const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * p.BN);
+          uint32_t accumulate = 0;
+          const int piece_end = kPieces ? min(i + p.piece_kb, tc.nkb) : tc.nkb;
+          for (; i < piece_end; ++i) {
+            tw0 = dbg ? clock64() : 0;
+            if (!peek && !__all_sync(kAll, mbar_wait_bounded(full_addr, ph, abort_flag, budget_ns))) {
+              if (el) record_error(p, abort_flag, kErrMmaWaitFull);
+              ok = false;
+              break;
+            }
+            if (dbg) dbg_wait_full += clock64() - tw0;
+            // probe the next ring slot now; the answer (a shared-memory round trip of about
+            // 100 cycles) is only read after this k-block's MMAs have been issued
+            const uint32_t nfull = (s + 1 == stages) ? full0 : full_addr + 8;
+            const uint32_t nph = (s + 1 == stages) ? (ph ^ 1u) : ph;
+            const uint32_t probe = mbar_test_wait(nfull, nph);
+            const uint32_t sfb_t = sfa_t + 4u * sfa_atoms;
+            tc_fence_after_sync();
+            if constexpr (kMx) {
+              // this k-block's scale atoms: shared -> the slot's tensor-memory columns
+              uint32_t src = sf_lo, dst = sfa_t;
+              for (uint32_t a = 0; a < sf_atoms; ++a, src += 32, dst += 4)
+                tmem_cp_atom_g<kPair>(dst, src, sf_hi, el);
+            }
+            if constexpr (KIND == kKindI8) {
+              mma_i8_g<kPair>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, accumulate, el);
+              mma_i8_g<kPair>(d_tmem, a_lo + a_k, a_hi, b_lo + b_k, b_hi, idesc, 1u, el);
+              mma_i8_g<kPair>(d_tmem, a_lo + 2 * a_k, a_hi, b_lo + 2 * b_k, b_hi, idesc, 1u, el);
+              mma_i8_g<kPair>(d_tmem, a_lo + 3 * a_k, a_hi, b_lo + 3 * b_k, b_hi, idesc, 1u, el);
+            } else if constexpr (KIND == kKindMxf8) {
+              mma_mxf8f6f4_g<kPair>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, sfa_t, sfb_t, accumulate, el);
+              mma_mxf8f6f4_g<kPair>(d_tmem, a_lo + 2, a_hi, b_lo + 2, b_hi, id1, sfa_t, sfb_t, 1u, el);
+              mma_mxf8f6f4_g<kPair>(d_tmem, a_lo + 4, a_hi, b_lo + 4, b_hi, id2, sfa_t, sfb_t, 1u, el);
+              mma_mxf8f6f4_g<kPair>(d_tmem, a_lo + 6, a_hi, b_lo + 6, b_hi, id3, sfa_t, sfb_t, 1u, el);
+            } else {
+              mma_mxf4_g<kPair>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, sfa_t, sfb_t, accumulate, el);
+              mma_mxf4_g<kPair>(d_tmem, a_lo + 2, a_hi, b_lo + 2, b_hi, id1, sfa_t, sfb_t, 1u, el);
+              mma_mxf4_g<kPair>(d_tmem, a_lo + 4, a_hi, b_lo + 4, b_hi, id2, sfa_t + sfa_half, sfb_t + sfb_half, 1u, el);
+              mma_mxf4_g<kPair>(d_tmem, a_lo + 6, a_hi, b_lo + 6, b_hi, id3, sfa_t + sfa_half, sfb_t + sfb_half, 1u, el);
+            }
+            accumulate = 1u;
+            tc_commit_both<kPair>(empty_addr, el);  // frees the stage (in both CTAs) once these MMAs have read it
+            peek = __all_sync(kAll, probe != 0) ? 1u : 0u;
+            if constexpr (kMx) {
+              sfa_t += sf_cols;
+              if (++sf_q == sf_slots) {
+                sf_q = 0;
+                sfa_t = sf_t0;
+              }
+            }
+            if (++s == stages) {
+              s = 0;
+              ph ^= 1u;
+              a_lo = a_lo0;
+              b_lo = b_lo0;
+              full_addr = full0;
+              empty_addr = empty0;
+              sf_lo = sf_lo0;
+            } else {
+              a_lo += stage_step;
+              b_lo += stage_step;
+              full_addr += 8;
+              empty_addr += 8;
+              sf_lo += sf_step;
             }
           }
-          if (++s == stages) {
-            s = 0;
-            ph ^= 1u;
-            a_lo = a_lo0;
-            b_lo = b_lo0;
-            full_addr = full0;
-            empty_addr = empty0;
-            sf_lo = sf_lo0;
-          } else {
-            a_lo += stage_step;
-            b_lo += stage_step;
-            full_addr += 8;
-            empty_addr += 8;
-            sf_lo += sf_step;
+          if (ok) tc_commit_both<kPair>(acc_full_bar(buf), el);
+          if (++buf == nacc) {
+            buf = 0;
+            acc_ph ^= 1u;
           }
-        }
-        if (ok) tc_commit_both<kPair>(acc_full_bar(buf), el);
-        if (++buf == nacc) {
-          buf = 0;
-          acc_ph ^= 1u;
-        }
+        } while (kPieces && ok && i < tc.nkb);
       }
       // Nothing may still be executing when tensor memory is released.
       tc_commit_g<kPair>(drain_bar, el);
