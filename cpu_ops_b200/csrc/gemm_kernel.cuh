@@ -946,7 +946,10 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
           } else if (d_rows) {
             __syncwarp();  // every lane's row is there
             write_d_rows(p, my_c + cq_b * 4096u, row0, kcol0, lane);
-            __syncwarp();  // every lane has read its words: the buffer may be written again
+            // every lane has read its words: the buffer may be written again, by TMA (which these
+            // plain accesses come before only through a proxy fence) if C arrives that way
+            if (c_tma) fence_proxy_async_shared_cta();
+            __syncwarp();
           } else if (ring) {
             __syncwarp();  // every lane has read its row: the buffer may be refilled
           }

@@ -81,6 +81,26 @@ def test_mixed_rings(gpu, m, n, k, pair, c_pad, d_pad):
     assert bool((D[:, n:] == 77).all())
 
 
+@pytest.mark.parametrize("m,n,k,pair", [(520, 771, 256, None), (4200, 4199, 512, True), (3000, 4097, 128, False)])
+def test_rows_beside_tma_in_place(gpu, m, n, k, pair):
+    """C == D with an aligned leading dimension and n not a multiple of four: C arrives by TMA in
+    the buffers that D leaves by rows, and every warp refills each buffer many times."""
+    ld = (n + 3) // 4 * 4
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    A = torch.randint(0, 256, (m, k), dtype=torch.uint8, device="cuda", generator=g)
+    B = torch.randint(-128, 128, (n, k), dtype=torch.int8, device="cuda", generator=g)
+    C = torch.randint(-1000, 1000, (m, ld), dtype=torch.int32, device="cuda", generator=g)
+    # |sums| < 2^53: exact in f64
+    want = (A.double() @ B.double().T).to(torch.int32) + C[:, :n]
+    gap = C[:, n:].clone()
+    op = c.GemmU8S8S32(c.RowMajor, c.ColumnMajor, c.RowMajor, pair=pair)
+    st = op(op.Arguments(c.GemmCoord(m, n, k), c.TensorRef(A, k), c.TensorRef(B, k), c.TensorRef(C, ld),
+                         c.TensorRef(C, ld), c.LinearCombination(1, 1)))
+    assert st == c.Status.kSuccess, _capi.last_error()
+    assert torch.equal(C[:, :n], want)
+    assert torch.equal(C[:, n:], gap)
+
+
 @pytest.mark.parametrize("fmt,k", [(_capi.FMT_E4M3, 200), (_capi.FMT_E2M1, 333), (_capi.FMT_E2M1, 1152)])
 @pytest.mark.parametrize("c_rm,shift", [(True, 0), (True, 1), (False, 1)])
 def test_mx(gpu, oracle, fmt, k, c_rm, shift):
