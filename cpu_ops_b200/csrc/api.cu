@@ -899,6 +899,10 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
     bool want = pair_pays(Mk, Nk, k_blocks, ch.BN, ch.slices, sms, bk_role_mn) ||
                 (ch.slices == 1 && d->tile_n == 0 &&
                  pair_pays_in_one_wave(Mk, Nk, k_blocks, ch.BN, sms, kind, beta_nonzero));
+    // Pairs sum k in one piece, and their scales are re-laid-out in front: a plan in pieces stays
+    // with one CTA per tile (e4m3 1024 x 704 x 20480 in five slices: pairs 43.8 us and 2.4e-6 off
+    // float64, 32 k-blocks to a sum; one CTA per tile 39.0 us, 22 to a sum).
+    if (ch.piece_kb < k_blocks) want = false;
     if (env_switches().pair >= 0) want = env_switches().pair != 0;
     if (d->flags & CPUOPS_B200_FLAG_PAIR_ON) want = true;
     if (d->flags & CPUOPS_B200_FLAG_PAIR_OFF) want = false;
