@@ -166,7 +166,8 @@ int pick_tile_width(int Mk, int Nk, int k_blocks, bool is_mx, int sms, bool beta
 
 struct DecodePlan {
   bool use = false;
-  int BN = 32, tiles = 0, grid = 0, stages = 0, splits = 1, tmem_cols = 128;
+  int BN = 32, tiles = 0, grid = 0, stages = 0, splits = 1, piece_kb = 0, tmem_cols = 128;
+  bool pieces = false;
   int smem = 0;
 };
 
@@ -187,9 +188,7 @@ int decode_clusters(DeviceState& st, int kind, int splits) {
     probe.attrs = attr;
     probe.numAttrs = 1;
     int n = 0;
-    const cudaError_t e = kind == kKindMxf4
-                              ? cudaOccupancyMaxActiveClusters(&n, decode_mx_kernel<kKindMxf4>, &probe)
-                              : cudaOccupancyMaxActiveClusters(&n, decode_mx_kernel<kKindMxf8>, &probe);
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, decode_kernel(kind, false), &probe);
     if (e != cudaSuccess) {
       cudaGetLastError();
       n = 0;
@@ -231,6 +230,15 @@ DecodePlan plan_decode(DeviceState& st, int kind, int Mk, int Nk, int k_blocks, 
   }
   const int units = dp.splits > 1 ? (k_blocks + dp.splits - 1) / dp.splits
                                   : (dp.tiles + dp.grid - 1) / dp.grid * k_blocks;  // most per CTA
+  // Few tiles are summed over no more k-blocks at a time than an SM's equal share of all of
+  // them (at least four), as if every SM had a piece of k of its own (kPieces in decode_kernel.cuh).
+  const int part = (k_blocks + dp.splits - 1) / dp.splits;
+  if (!never_split && 4 * dp.tiles < cap) {
+    const int longest = std::max(4, static_cast<int>(static_cast<int64_t>(dp.tiles) * k_blocks / cap));
+    const int pieces = (part + longest - 1) / longest;
+    dp.piece_kb = (part + pieces - 1) / pieces;
+    dp.pieces = pieces > 1;
+  }
   // the deepest ring the shared memory allows: the stream needs the bytes in flight
   int stages = (st.smem_optin - 1024 - decode_staging_bytes(dp.BN) - decode_reduce_bytes(Nk, dp.splits) - kDecodeBarrierBytes) /
                per_stage;
@@ -241,7 +249,7 @@ DecodePlan plan_decode(DeviceState& st, int kind, int Mk, int Nk, int k_blocks, 
   // one CTA per SM must not be joined by a second one of the same launch
   dp.smem = std::max(dp.smem, 120 * 1024);
   const int sf_cols = 4 * 2 * ka;
-  int cols = 2 * dp.BN + kDecodeSfSlots * sf_cols;
+  int cols = (dp.pieces ? 3 : 2) * dp.BN + kDecodeSfSlots * sf_cols;
   dp.tmem_cols = 32;
   while (dp.tmem_cols < cols) dp.tmem_cols *= 2;
   return dp;
@@ -1127,6 +1135,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
     q.BN = dp.BN;
     q.stages = dp.stages;
     q.splits = dp.splits;
+    q.piece_kb = dp.piece_kb;
     q.tmem_cols = dp.tmem_cols;
     if (kind == kKindMxf4) {
       q.idesc = make_idesc_block_scaled(1u, 1u, kTileM, dp.BN);  // e2m1 x e2m1
@@ -1151,11 +1160,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
       if (!told) {
         told = true;
         int per_sm = 0;
-        if (kind == kKindMxf4) {
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_mx_kernel<kKindMxf4>, kDecodeThreads, dp.smem);
-        } else {
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_mx_kernel<kKindMxf8>, kDecodeThreads, dp.smem);
-        }
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_kernel(kind, dp.pieces), kDecodeThreads, dp.smem);
         fprintf(stderr, "[instrument] decode kernel: %d bytes of shared memory, %d CTAs per SM can be resident\n",
                 dp.smem, per_sm);
       }
@@ -1192,11 +1197,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
     g_last_plan.grid = dp.grid;
     g_last_plan.epilogue_warps = 4;
     g_last_plan.decode = 1;
-    if (kind == kKindMxf4) {
-      CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_mx_kernel<kKindMxf4>, tmW, tmX, q));
-    } else {
-      CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_mx_kernel<kKindMxf8>, tmW, tmX, q));
-    }
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_kernel(kind, dp.pieces), tmW, tmX, q));
     g_launches.fetch_add(1);
     CUDA_TRY(cudaGetLastError());
     if (profile) {

@@ -21,6 +21,12 @@
 //     owner's buffer, its barrier counting the bytes), and each owner adds the pieces of its
 //     part in ascending k order - a fixed order, so results do not depend on which CTA
 //     finished first.  The cut of a tile never leaves the chip and needs no workspace.
+//   * A CTA's part of k may be summed in pieces (kPieces).  The tensor cores drop the low bits of a running
+//     sum: against float64, 8-bit results are off by 6e-10 per element of k summed in one
+//     accumulator.  Where few tiles leave every CTA a long part, the two accumulators take turns every
+//     p.piece_kb k-blocks and the epilogue warps add them up in f32, in ascending k order, in tensor
+//     memory beside them, while the MMAs of the next piece run.  m = 32, 1024 weight rows x k =
+//     14336, e4m3: 1.4e-6 off in one sum of 19 k-blocks, 4.1e-7 in pieces of 5; 9.3 us / 9.6.
 //   * Launched with programmatic stream serialization: a CTA may become resident and set up
 //     its barriers and tensor memory while the kernel before this one in the stream is
 //     still finishing; every role then waits (griddepcontrol.wait) before it reads or
@@ -72,7 +78,8 @@ struct DecodeParams {
   int32_t BN;                // 32 or 64
   int32_t stages;
   int32_t splits;            // CTAs (one cluster) that share a tile's k; 1: whole tiles per CTA
-  int32_t tmem_cols;         // power of two >= 2 * BN + kDecodeSfSlots * scale columns per unit
+  int32_t piece_kb;          // kPieces: k-blocks summed in one accumulator
+  int32_t tmem_cols;         // power of two >= 2 (kPieces: 3) * BN + kDecodeSfSlots * scale columns per unit
   uint32_t idesc;
   uint32_t wait_budget_us;   // budget of every bounded wait
   EpilogueParams epi;
@@ -145,7 +152,11 @@ __device__ __forceinline__ uint32_t pick_word(const uint4& v, int i) {
   return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
 }
 
-template <int KIND>
+__device__ __forceinline__ uint32_t add_f32(uint32_t a, uint32_t b) {
+  return __float_as_uint(__fadd_rn(__uint_as_float(a), __uint_as_float(b)));
+}
+
+template <int KIND, bool kPieces>
 __global__ void __launch_bounds__(kDecodeThreads, 1)
     decode_mx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                      const DecodeParams p) {
@@ -292,8 +303,9 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
     uint32_t ph = 0, acc_ph = 0;
     bool ok = true;
     int i = 0;
+    [[maybe_unused]] int tile_left = kb1 - kb0;
     while (i < n_units && ok) {
-      const int piece_units = kb1 - kb0;  // one tile
+      const int piece_units = kPieces ? min(tile_left, p.piece_kb) : kb1 - kb0;  // ... or one tile
       if (!__all_sync(kAll, mbar_wait_bounded(acc_empty_bar(buf), acc_ph ^ 1u, abort_flag, budget_ns))) {
         if (el) {
           leave_error(p.error, kErrMmaWaitAcc);
@@ -344,6 +356,10 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       tc_commit_g<false>(acc_full_bar(buf), el);
       if (++buf == 2) { buf = 0; acc_ph ^= 1u; }
       i += piece_units;
+      if constexpr (kPieces) {
+        tile_left -= piece_units;
+        if (tile_left == 0) tile_left = kb1 - kb0;
+      }
     }
     // nothing may still be executing when tensor memory is released
     tc_commit_g<false>(drain_bar, el);
@@ -465,8 +481,45 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
     uint32_t acc_ph = 0;
     bool alive = true;
     if (splits > 1) cluster_wait();
+    // kPieces: the sum of a tile's finished pieces, behind the accumulators and the scale slots
+    const uint32_t tsum =
+        tmem_base + (static_cast<uint32_t>(q * 32) << 16) + 2u * static_cast<uint32_t>(BN) + kDecodeSfSlots * kSfCols;
     for (int tile = tile0; tile < tile1; ++tile) {
-      const bool got = mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
+      // the accumulator is in registers: hand the buffer back to the MMA warp
+      auto hand_back = [&]() {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty_bar(buf));
+      };
+      [[maybe_unused]] bool summed = false;
+      if constexpr (kPieces) {  // all pieces of this CTA's part of k but the last
+        for (int left = kb1 - kb0; left > p.piece_kb && alive; left -= p.piece_kb) {
+          const bool ready = mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
+          if (!__all_sync(0xffffffffu, ready)) {
+            alive = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t from = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
+#pragma unroll 1
+          for (int c = 0; c < p.Nk; c += 16) {
+            uint32_t v[16], w[16];
+            tmem_ld_32x16(from + static_cast<uint32_t>(c), v);
+            if (summed) tmem_ld_32x16(tsum + static_cast<uint32_t>(c), w);
+            tmem_ld_wait();
+            if (summed) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = add_f32(w[j], v[j]);
+            }
+            tmem_st_32x16(tsum + static_cast<uint32_t>(c), v);
+          }
+          tmem_st_wait();
+          hand_back();
+          if (++buf == 2) { buf = 0; acc_ph ^= 1u; }
+          summed = true;
+        }
+      }
+      const bool got = alive && mbar_wait_bounded(acc_full_bar(buf), acc_ph, abort_flag, budget_ns);
       if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) {
           leave_error(p.error, kErrEpilogueWait);
@@ -479,13 +532,22 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       if (tile + 1 == tile1) DECODE_STAMP(p, 6, warp == 6 && lane == 0);
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
       const int krow = tile * kTileM + q * 32 + lane;
-      // the accumulator is in registers: hand the buffer back to the MMA warp
-      auto hand_back = [&]() {
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty_bar(buf));
+      // a chunk of the finished sum: the last piece's accumulator, with what the others left
+      auto load16 = [&](int c, uint32_t (&r)[16]) {
+        tmem_ld_32x16(taddr + static_cast<uint32_t>(c), r);
+        if constexpr (kPieces) {
+          if (summed) {
+            uint32_t w[16];
+            tmem_ld_32x16(tsum + static_cast<uint32_t>(c), w);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] = add_f32(w[j], r[j]);
+            return;
+          }
+        }
+        tmem_ld_wait();
       };
-      if (splits == 1 && p.Nk > 16) {
+      if (splits == 1 && p.Nk > 16 && !kPieces) {
         for (int c = 0; c < p.Nk; c += 32) {
           uint32_t r[32];
           tmem_ld_32x32(taddr + static_cast<uint32_t>(c), r);
@@ -493,10 +555,17 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
           if (c + 32 >= p.Nk) hand_back();
           if (krow < p.Mk) decode_store_chunk<32>(e, r, krow, c, min(32, p.Nk - c));
         }
+      } else if (splits == 1 && kPieces) {
+#pragma unroll 1
+        for (int c = 0; c < p.Nk; c += 16) {
+          uint32_t r[16];
+          load16(c, r);
+          if (c + 16 >= p.Nk) hand_back();
+          if (krow < p.Mk) decode_store_chunk<16>(e, r, krow, c, min(16, p.Nk - c));
+        }
       } else if (splits == 1) {
         uint32_t r[16];
-        tmem_ld_32x16(taddr, r);
-        tmem_ld_wait();
+        load16(0, r);
         if (tile + 1 == tile1) DECODE_STAMP(p, 8, warp == 6 && lane == 0);
         hand_back();
         if (krow < p.Mk) decode_store_chunk<16>(e, r, krow, 0, p.Nk);
@@ -504,8 +573,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1)
       } else {
         for (int c = 0; c < nchunks; ++c) {
           uint32_t r[16];
-          tmem_ld_32x16(taddr + static_cast<uint32_t>(c * 16), r);
-          tmem_ld_wait();
+          load16(c * 16, r);
           // this lane's 64 bytes of the unit, 16-byte pieces XOR-swizzled over pairs of lanes
           // (rows are 64 bytes apart: without it every other lane would meet the same banks)
           const int u = q + 4 * c, owner = u % splits, slot = u / splits;

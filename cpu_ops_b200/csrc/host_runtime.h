@@ -172,6 +172,13 @@ GemmKernel gemm_kernel(int kind, bool pair, bool raw_scales) {
   return pair ? gemm_tcgen05_kernel<kKindMxf4, true> : gemm_tcgen05_kernel<kKindMxf4, false>;
 }
 
+// The decode kernel's.
+using DecodeKernel = void (*)(CUtensorMap, CUtensorMap, DecodeParams);
+DecodeKernel decode_kernel(int kind, bool pieces) {
+  if (kind == kKindMxf4) return pieces ? decode_mx_kernel<kKindMxf4, true> : decode_mx_kernel<kKindMxf4, false>;
+  return pieces ? decode_mx_kernel<kKindMxf8, true> : decode_mx_kernel<kKindMxf8, false>;
+}
+
 DeviceState g_dev[64];
 EncodeTiledFn g_encode = nullptr;
 int g_device_count = -2;  // -2: not probed; guarded by g_registry_mu
@@ -269,10 +276,10 @@ int init_device(int device, DeviceState** out) {
         for (int form = 0; form < 3; ++form)
           CUDA_TRY(cudaFuncSetAttribute(gemm_kernel(kind, form == 1, form == 2),
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
-      CUDA_TRY(cudaFuncSetAttribute(decode_mx_kernel<kKindMxf8>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
-      CUDA_TRY(cudaFuncSetAttribute(decode_mx_kernel<kKindMxf4>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
+      for (int kind : {kKindMxf8, kKindMxf4})
+        for (bool pieces : {false, true})
+          CUDA_TRY(cudaFuncSetAttribute(decode_kernel(kind, pieces), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        st.smem_optin));
       st.ready.store(true, std::memory_order_release);
     }
   }

@@ -44,6 +44,10 @@ def bound(elements):
     return 2e-7 + 6.3e-10 * elements
 
 
+def bound_e2m1(elements):  # (fewer of the products' bits fall off the end)
+    return 1.2e-7 + 2.5e-10 * elements
+
+
 # 160 k-blocks, once cut in seven (23 k-blocks at most), now in five slices of 32 and pieces of 22
 @pytest.mark.parametrize("fmt,m,n,lo", [(F8, 1024, 704, 114), (F5, 2560, 256, 108), (F8, 1792, 384, 114)])
 def test_a_plan_in_pieces_stays_with_one_cta_per_tile(gpu, fmt, m, n, lo):
@@ -51,3 +55,23 @@ def test_a_plan_in_pieces_stays_with_one_cta_per_tile(gpu, fmt, m, n, lo):
     e = error(fmt, m, n, 20480, 640, lo, lo + 6)
     assert _capi.last_plan().pair == 0
     assert e <= bound(23 * 128), e
+
+
+# Once a CTA per SM shared the tiles' k-blocks evenly; now at most six share a tile and sum their part in
+# pieces.  `longest`: k-blocks to a sum then.  One and four 16-column chunks, whole tiles and clusters.
+@pytest.mark.parametrize("fmt,lo,m,n,k,longest", [
+    (F8, 114, 32, 1024, 14336, 7), (F8, 114, 1, 512, 14336, 4), (F8, 114, 17, 1024, 8192, 4), (F5, 108, 64, 1536, 14336, 10),
+    (F8, 114, 64, 4608, 14336, 28), (F8, 114, 8, 1000, 1024, 4), (F8, 114, 40, 1000, 1024, 4), (F8, 114, 33, 130, 2080, 4),
+    (F8, 114, 32, 1024, 65536, 28)])
+def test_decode_8_bit(gpu, fmt, lo, m, n, k, longest):
+    e = error(fmt, m, n, k, -(-k // 512) * 16, lo, lo + 6)
+    assert _capi.last_plan().decode == 1
+    assert e <= bound(longest * 128), e
+
+
+# Scales over 15 exponents: sums of e2m1 products no longer fit f32.
+@pytest.mark.parametrize("m,n,k,longest", [(32, 1024, 28672, 7), (1, 512, 28672, 4), (64, 1000, 16384, 4), (16, 1000, 2048, 4)])
+def test_decode_4_bit(gpu, m, n, k, longest):
+    e = error(F4, m, n, k, -(-k // 512) * 16, 120, 134)
+    assert _capi.last_plan().decode == 1
+    assert e <= bound_e2m1(longest * 256), e
