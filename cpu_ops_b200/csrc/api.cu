@@ -433,7 +433,9 @@ static int launch_relayout(const void* src0, void* dst0, const ScaleLayout& L0, 
 static int launch_reduce(bool is_mx, const EpilogueParams& epi, const uint32_t* ws, int slices, int Mk, int Nk, int sms,
                          cudaStream_t stream) {
   const int threads = 256;
-  const int64_t tiles = static_cast<int64_t>((Mk + 31) / 32) * ((Nk + 7) / 8);
+  // (a few 32 x 32 tiles per SM at least, see reduce_epilogue_kernel)
+  const bool wide = static_cast<int64_t>((Mk + 31) / 32) * ((Nk + 31) / 32) >= 4 * sms;
+  const int64_t tiles = static_cast<int64_t>((Mk + 31) / 32) * (wide ? (Nk + 31) / 32 : (Nk + 7) / 8);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(std::min<int64_t>(tiles, static_cast<int64_t>(sms) * 16)));
   cfg.blockDim = dim3(threads);
@@ -443,11 +445,9 @@ static int launch_reduce(bool is_mx, const EpilogueParams& epi, const uint32_t* 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = env_switches().no_pdl || g_profile.load() ? 0 : 1;
-  if (is_mx) {
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_epilogue_kernel<false>, epi, ws, slices, Mk, Nk));
-  } else {
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_epilogue_kernel<true>, epi, ws, slices, Mk, Nk));
-  }
+  auto* kernel = is_mx ? (wide ? reduce_epilogue_kernel<false, 32> : reduce_epilogue_kernel<false, 8>)
+                       : (wide ? reduce_epilogue_kernel<true, 32> : reduce_epilogue_kernel<true, 8>);
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, epi, ws, slices, Mk, Nk));
   g_launches.fetch_add(1);
   CUDA_TRY(cudaGetLastError());
   return 0;

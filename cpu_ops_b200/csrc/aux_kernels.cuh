@@ -139,54 +139,72 @@ __global__ void relayout_scales_kernel(const uint8_t* __restrict__ src0, uint8_t
 // (gemm/kernel/run_blocked.h:40-75); slices == 0 is its write_zero_k (:30-36).
 // A slab is stored column by column (the accumulator's lanes are rows, so the GEMM writes
 // 128 contiguous bytes per instruction; by rows of D it wrote 16 bytes to each of 32 lines).
-// A block reads 32 rows x 8 columns of every slab - one element per thread, its words of eight
-// slabs in flight - and turns them in shared memory where D's rows are contiguous.  Bound by
-// the latency of those reads and by the gap between two launches, which programmatic stream
-// serialization hides: 192 x 320 x 16384 u8 x s8 in 22 slices, both kernels, 13.5 -> 12.4 us.
-template <bool kInt>
+// A block reads 32 rows x kCols columns of every slab - kCols / 8 elements per thread, the words of several
+// slabs in flight - and turns them in shared memory where D's rows are contiguous.  Small outputs take
+// kCols = 8, many blocks: bound by the latency of those reads and by the gap between two launches, which
+// programmatic stream serialization hides: 192 x 320 x 16384 u8 x s8 in 22 slices, both kernels,
+// 13.5 -> 12.4 us.  Large ones take 32: with 8 a row of D is written 32 bytes at a time (GEMM and reduction,
+// kCols = 8 / 32: 640 x 1024 x 16384 in 3 slices 20.9 / 18.2 us, 1024 x 2048 x 16384 in 4 53.1 / 42.2,
+// 2048 x 2048 x 8192 in 2 76.7 / 55.7; 1000 x 300 x 8192 e4m3 in 8 20.9 / 22.5, too few blocks).
+template <bool kInt, int kCols>
 __global__ void __launch_bounds__(256) reduce_epilogue_kernel(EpilogueParams e, const uint32_t* ws, int slices, int Mk,
                                                               int Nk) {
-  __shared__ uint32_t turn[8][33];
+  constexpr int kPer = kCols / 8;           // columns per warp
+  constexpr int kFlight = kPer == 1 ? 8 : 4;  // slabs whose words are in flight together
+  __shared__ uint32_t turn[kCols][33];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int row_tiles = (Mk + 31) / 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t tiles = static_cast<int64_t>(row_tiles) * ((Nk + 7) / 8), slab = static_cast<int64_t>(Mk) * Nk;
+  const int64_t tiles = static_cast<int64_t>(row_tiles) * ((Nk + kCols - 1) / kCols), slab = static_cast<int64_t>(Mk) * Nk;
   const bool by_rows = e.d_sr != 1;
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the slabs are written
   for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const int row0 = static_cast<int>(t % row_tiles) * 32, col0 = static_cast<int>(t / row_tiles) * 8;
-    int krow = row0 + lane, kcol = col0 + warp;
-    uint32_t acc = 0;
-    if (slices > 0 && krow < Mk && kcol < Nk) {
-      const uint32_t* w = ws + (static_cast<int64_t>(kcol) * Mk + krow);
-      for (int s0 = 0; s0 < slices; s0 += 8) {
-        uint32_t v[8];
+    const int row0 = static_cast<int>(t % row_tiles) * 32, col0 = static_cast<int>(t / row_tiles) * kCols;
+    uint32_t acc[kPer];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = s0 + j < slices ? __ldcg(w + (s0 + j) * slab) : 0u;
+    for (int c = 0; c < kPer; ++c) acc[c] = 0;
+    if (slices > 0 && row0 + lane < Mk) {
+      const uint32_t* w = ws + (static_cast<int64_t>(col0 + warp) * Mk + row0 + lane);
+      for (int s0 = 0; s0 < slices; s0 += kFlight) {
+        uint32_t v[kFlight][kPer];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < kFlight; ++j)
+#pragma unroll
+          for (int c = 0; c < kPer; ++c)
+            v[j][c] = s0 + j < slices && col0 + warp + 8 * c < Nk ? __ldcg(w + (s0 + j) * slab + static_cast<int64_t>(8 * c) * Mk) : 0u;
+#pragma unroll
+        for (int j = 0; j < kFlight; ++j) {
           if (s0 + j >= slices) break;
-          if (s0 + j == 0) {
-            acc = v[0];
-          } else if constexpr (kInt) {
-            acc += v[j];
-          } else {
-            acc = __float_as_uint(__fadd_rn(__uint_as_float(acc), __uint_as_float(v[j])));
+#pragma unroll
+          for (int c = 0; c < kPer; ++c) {
+            if (s0 + j == 0) {
+              acc[c] = v[0][c];
+            } else if constexpr (kInt) {
+              acc[c] += v[j][c];
+            } else {
+              acc[c] = __float_as_uint(__fadd_rn(__uint_as_float(acc[c]), __uint_as_float(v[j][c])));
+            }
           }
         }
       }
     }
     if (by_rows) {
-      turn[warp][lane] = acc;
+#pragma unroll
+      for (int c = 0; c < kPer; ++c) turn[warp + 8 * c][lane] = acc[c];
       __syncthreads();
-      krow = row0 + static_cast<int>(threadIdx.x >> 3);
-      kcol = col0 + static_cast<int>(threadIdx.x & 7);
-      acc = turn[threadIdx.x & 7][threadIdx.x >> 3];
-      __syncthreads();  // (the next tile overwrites it)
     }
-    if (krow < Mk && kcol < Nk) {
-      const uint32_t out = epilogue_element<kInt>(e, acc, krow, kcol);
-      static_cast<uint32_t*>(e.D)[krow * e.d_sr + kcol * e.d_sc] = out;
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      int krow = row0 + lane, kcol = col0 + warp + 8 * c;
+      if (by_rows) {
+        const int i = static_cast<int>(threadIdx.x) + 256 * c;
+        krow = row0 + i / kCols;
+        kcol = col0 + i % kCols;
+        acc[c] = turn[i % kCols][i / kCols];
+      }
+      if (krow < Mk && kcol < Nk)
+        static_cast<uint32_t*>(e.D)[krow * e.d_sr + kcol * e.d_sc] = epilogue_element<kInt>(e, acc[c], krow, kcol);
     }
+    if (by_rows) __syncthreads();  // (the next tile overwrites it)
   }
 }
 
