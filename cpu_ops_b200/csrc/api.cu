@@ -429,12 +429,16 @@ static int launch_relayout(const void* src0, void* dst0, const ScaleLayout& L0, 
   return 0;
 }
 
+// Whether the split-k reduction takes 32 x 32 tiles (see reduce_epilogue_kernel): a few per SM at least.
+static bool wide_reduction(int Mk, int Nk, int sms) {
+  return static_cast<int64_t>((Mk + 31) / 32) * ((Nk + 31) / 32) >= 4 * sms;
+}
+
 // D = epilogue(the slabs' sum, C); no slabs: k == 0.
 static int launch_reduce(bool is_mx, const EpilogueParams& epi, const uint32_t* ws, int slices, int Mk, int Nk, int sms,
                          cudaStream_t stream) {
   const int threads = 256;
-  // (a few 32 x 32 tiles per SM at least, see reduce_epilogue_kernel)
-  const bool wide = static_cast<int64_t>((Mk + 31) / 32) * ((Nk + 31) / 32) >= 4 * sms;
+  const bool wide = wide_reduction(Mk, Nk, sms);
   const int64_t tiles = static_cast<int64_t>((Mk + 31) / 32) * (wide ? (Nk + 31) / 32 : (Nk + 7) / 8);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(std::min<int64_t>(tiles, static_cast<int64_t>(sms) * 16)));
@@ -812,35 +816,52 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
       return CPUOPS_B200_STATUS_INVALID_ARGUMENTS;
     }
     // Few tiles and a deep k: cut k so that the work items fill the SMs.  Estimate in
-    // microseconds, fitted to calls on 64 x 128 .. 1024 x 1024 outputs with k = 4096 .. 32768 in 1
-    // to 24 slices: waves x k-blocks per slice x 0.13 (BN 128; 8-bit MX 0.21), and when split
-    // the second launch and the slabs, 1 + 9 per million outputs + 0.17 per slice (8-bit MX
-    // 2 more where its scales have to be re-laid-out).  Chosen by an estimate that charged every
-    // CTA an SM's share of HBM, before / now: u8 x s8 192 x 320 x 16384 (22 / 8 slices) 12.4 / 9.7 us,
-    // 640 x 1024 x 8192 (3 / 1) 17.5 / 15.7, 1024 x 1024 x 8192 (2 / 1) 23.0 / 18.4.
-    auto estimate = [&](int BN, int* slices) {
+    // microseconds: waves x k-blocks per slice x the time of a k-block, the epilogue (0.016 per
+    // column), and when split the second launch and the slabs: 1.3 + 7.5 per million outputs (4 in the
+    // reduction's wide form) + 0.18 and 0.4 per million outputs for each slice.  Over 64 k-blocks a k-block took,
+    // by tile width 64 / 128 / 160 / 256 and alike for 8 to 144 CTAs, 0.14 / 0.17 / 0.20 / 0.31 us for u8 x s8,
+    // 0.22 / 0.25 / 0.28 / 0.41 for 8-bit MX and 0.23 / 0.27 / 0.28 / 0.44 for e2m1; about a third more once A and B
+    // are as large as one die's half of L2.  With half that time for a k-block, and 64-wide tiles whenever k was cut
+    // for precision, calls had become slower than in the plans before: e4m3 640 x 1024 x 32768 62.0 us (36.4 before,
+    // 33.7 now), 512 x 1024 x 16384 28.8 (22.8, 22.4); u8 x s8 1024 x 1024 x 32768 52.6 (39.1, 37.3), 640 x 1024 x
+    // 16384 24.6 (20.7, 18.3); e2m1 640 x 1024 x 32768 40.4 (26.9, 23.6).
+    auto cost = [&](int BN, int s, int piece_kb) {
       const int n_tiles = (Nk + BN - 1) / BN, m_tiles = (Mk + 127) / 128, last = last_tile_width(Nk, BN);
       const int64_t tiles = static_cast<int64_t>(m_tiles) * n_tiles;
-      const double block_us = (kind == kKindMxf8 ? 0.21 : 0.13) * (128.0 + BN) / 256.0;
-      const double split_us = 1.0 + 9e-6 * Mk * static_cast<double>(Nk) + (kind == kKindMxf8 && !scale_rows_aligned(4) ? 2.0 : 0.0);
-      double best = 1e300;
+      const int per_slice = (k_blocks + s - 1) / s;
+      const double outputs_m = 1e-6 * Mk * static_cast<double>(Nk);
+      const double block_us = ((kind == kKindI8 ? 0.13 : kind == kKindMxf8 ? 0.20 : 0.215) +
+                               (kind == kKindI8 ? 2.7e-6 : 3.2e-6) * BN * BN) *
+                              (1.0 + 0.3 * std::min(1.0, 128.0 * (static_cast<double>(Mk) + Nk) * k_blocks / 64e6));
+      double rounds = static_cast<double>((tiles * s + sms - 1) / sms);
       // unsplit, a ragged last tile column is computed narrower and dealt out evenly:
       // rounds in units of a wide tile (feed-bound cost ~ 128 + width rows per k-block)
-      double rounds1 = static_cast<double>((tiles + sms - 1) / sms);
-      if (!bk_role_mn && n_tiles >= 2 && last < BN && !env_switches().no_narrow)
-        rounds1 = busiest_worker(m_tiles * (n_tiles - 1), m_tiles, sms, 1.0, (128.0 + last) / (128.0 + BN));
-      const bool may_split = d->split_k_slices == 0 && tiles < 2 * sms && k_blocks >= 8;
-      for (int s = 1; s <= (may_split ? std::min(32, k_blocks / 2) : 1); ++s) {
-        const int64_t waves = (tiles * s + sms - 1) / sms;
-        const int per_slice = (k_blocks + s - 1) / s;
-        double t_us = (s == 1 ? rounds1 : static_cast<double>(waves)) * per_slice * block_us;
-        if (s > 1) t_us += split_us + 0.17 * s;
-        if (t_us < best * 0.97) {
-          best = t_us;
-          *slices = s;
+      if (s == 1 && !bk_role_mn && n_tiles >= 2 && last < BN && !env_switches().no_narrow)
+        rounds = busiest_worker(m_tiles * (n_tiles - 1), m_tiles, sms, 1.0, (128.0 + last) / (128.0 + BN));
+      double us = rounds * per_slice * block_us + 0.016 * BN;
+      if (s > 1) us += 1.3 + (wide_reduction(Mk, Nk, sms) ? 4.0 : 7.5) * outputs_m + (0.18 + 0.4 * outputs_m) * s;
+      // the launch that re-lays the scales out (see raw_scales below; as if their rows were always aligned, so
+      // that the sums do not depend on it)
+      if (is_mx &&
+          !(fp4_pair ? tiles * s < 2 * sms : tiles * s <= sms || (s == 1 && tiles * k_blocks <= 32 * static_cast<int64_t>(sms))))
+        us += 2.5;
+      // pieces: about 0.03 per k-block and 0.25 per piece
+      if (piece_kb < per_slice) us += rounds * (0.03 * per_slice + 0.25 * ((per_slice - 1) / piece_kb));
+      return us;
+    };
+    auto best_slices = [&](int BN, int piece_kb) {
+      const int64_t tiles = static_cast<int64_t>((Mk + 127) / 128) * ((Nk + BN - 1) / BN);
+      int slices = 1;
+      if (d->split_k_slices != 0 || tiles >= 2 * sms || k_blocks < 8) return slices;
+      double best = cost(BN, 1, piece_kb);
+      for (int s = 2; s <= std::min(32, k_blocks / 2); ++s) {
+        const double us = cost(BN, s, piece_kb);
+        if (us < best * 0.97) {
+          best = us;
+          slices = s;
         }
       }
-      return best;
+      return slices;
     };
     // 8-bit MX: how many parts k would be cut into if every CTA had only an SM's share of HBM
     // bandwidth to feed it.  The tensor cores lose low bits along a running sum, so this is
@@ -870,28 +891,30 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
       ch.slices = std::min(d->split_k_slices, k_blocks);
     } else {
       const int parts = kind == kKindMxf8 && d->split_k_slices == 0 ? precision_parts(ch.BN) : 1;
+      const int piece_kb = parts > 1 ? std::max(1, k_blocks / parts) : ch.piece_kb;
       // a caller that asks for one of the two forms gets the same tile, slices and bits in either
       const bool form_given = (d->flags & (CPUOPS_B200_FLAG_PAIR_ON | CPUOPS_B200_FLAG_PAIR_OFF)) != 0;
-      const double us = estimate(ch.BN, &ch.slices);
-      // 64-wide tiles where even those run all at once: twice the CTAs, each with half the epilogue
-      // (about 0.016 us per column).  BN 128 / 64: u8 x s8 512^3 6.2 / 5.1 us, 1024^3 6.7 / 5.8, 128 x
+      if (parts > 1 && (ch.BN > 64 || form_given)) {  // (pairs sum k in one piece)
+        ch.slices = parts;
+      } else {
+        ch.slices = best_slices(ch.BN, piece_kb);
+        ch.piece_kb = piece_kb;
+      }
+      // 64-wide tiles where even those run all at once: twice the CTAs, each with half the epilogue,
+      // and narrow enough for pieces.  BN 128 / 64: u8 x s8 512^3 6.2 / 5.1 us, 1024^3 6.7 / 5.8, 128 x
       // 4096 x 4096 10.7 / 8.9, 300 x 1000 x 2000 11.0 / 8.8; e4m3 512 x 2048 x 1024 + bias + SiLU 11.2 /
-      // 9.6, 128 x 4096 x 4096 14.3 / 12.2; e2m1 512 x 2048 x 1024 7.6 / 7.0.
+      // 9.6, 128 x 4096 x 4096 14.3 / 12.2; e2m1 512 x 2048 x 1024 7.6 / 7.0.  Over a long k
+      // wide tiles in slices end sooner.
       const int64_t narrow_tiles = static_cast<int64_t>((Mk + 127) / 128) * ((Nk + 63) / 64);
       if (d->tile_n == 0 && !bk_role_mn && ch.BN > 64 && narrow_tiles <= sms && !form_given) {
-        int slices = 1;
-        if (estimate(64, &slices) + 0.016 * 64 < us + 0.016 * ch.BN || parts > 1) {
+        const int slices = best_slices(64, piece_kb);
+        if (cost(64, slices, piece_kb) < cost(ch.BN, ch.slices, k_blocks)) {
           ch.BN = 64;
           ch.slices = slices;
+          ch.piece_kb = piece_kb;
         }
       }
-      if (parts > 1) {
-        if (ch.BN <= 64 && !form_given) {  // (pairs sum k in one piece)
-          ch.piece_kb = std::max(1, k_blocks / parts);
-        } else {
-          ch.slices = parts;
-        }
-      }
+      if ((k_blocks + ch.slices - 1) / ch.slices <= ch.piece_kb) ch.piece_kb = k_blocks;  // (one piece a slice)
     }
     ch.nacc = (is_mx && ch.BN > 224) ? 1 : 2;
   }
