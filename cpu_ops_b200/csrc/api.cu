@@ -94,15 +94,16 @@ bool pair_pays(int Mk, int Nk, int k_blocks, int BN, int slices, int sms, bool b
 // SM where a CTA stages 48 KB, so a long k loop wins.  One CTA per tile / pairs, both with
 // eight epilogue warps: u8 x s8 2048^3 beta = 1 (16 k-blocks) 17.3 / 16.8 us, beta = 0 14.2 / 14.5,
 // 1536 x 2816 x 1024 (8) 14.0 / 14.6, 1024 x 4096 x 4096 (32) 22.7 / 20.1, 2048 x 2304 x 8192
-// (64) 37.3 / 30.4; e4m3 2048^3 (16) 21.0 / 21.2, 1024 x 4096 x 4096 (32) 27.3 / 26.9,
-// 2048 x 2304 x 8192 (64) 47.2 / 43.7; e2m1 2048^3 (8) 17.4 / 18.0, 2048 x 2304 x 8192 (32)
-// 32.1 / 31.4.  At 16 k-blocks only the C that is read beside them decides.
-// e2m1 has its raw scales in the one-CTA form only (kRaw), which is worth more: 25.6 us.
+// (64) 37.3 / 30.4.  At 16 k-blocks only the C that is read beside them decides.  (These with operands from HBM;
+// with operands in L2 u8 x s8 2048 x 2304 x 4096 takes 18.7 / 20.4, x 8192 29.2 / 29.0.)
+// MX has its raw scales in the one-CTA form only (kRaw), which is worth more until k is long:
+// e4m3 1024 x 4096 x 4096 (32) 22.4 to 23.6 / 24.1, 2048 x 2304 x 4096 (32) 25.0 / 31.7, x 8192 (64) 39.6 / 39.5,
+// x 16384 (128) 79.4 / 70.9; e2m1 2048 x 2304 x 8192 (32) 25.6 / 31.4, never pairs.
 bool pair_pays_in_one_wave(int Mk, int Nk, int k_blocks, int BN, int sms, int kind, bool beta) {
   const int64_t pairs = static_cast<int64_t>((Mk + 255) / 256) * ((Nk + BN - 1) / BN);
   const bool halves_full = (Mk + 127) / 128 % 2 == 0;
   return BN == 256 && Mk > 128 && halves_full && 2 * pairs <= sms && kind != kKindMxf4 &&
-         k_blocks >= (kind == kKindI8 && beta ? 16 : 24);
+         k_blocks >= (kind == kKindMxf8 ? 96 : beta ? 16 : 24);
 }
 
 // Estimated SM cycles of an unsplit launch with tile width BN.  Per k-block a CTA is bound

@@ -4,7 +4,8 @@ import pytest
 import torch
 
 import cpu_ops_b200 as c
-from cpu_ops_b200 import _capi
+from cpu_ops_b200 import _capi, workloads as W
+from tests.gpu_helpers import STORAGE
 
 pytestmark = pytest.mark.gpu
 
@@ -26,6 +27,25 @@ def test_pairs_in_one_wave(gpu, m, n, k, beta, pair):
         assert _capi.last_plan().pair == pair
     # |sums| < 2^53: exact in f64
     assert torch.equal(D, (A.double() @ B.double().T).to(torch.int32) + beta * C)
+
+
+@pytest.mark.parametrize("k,pair", [(4096, 0), (12160, 0), (12288, 1)])
+def test_mx_pairs_in_one_wave(gpu, k, pair):
+    """One CTA per tile reads the scales itself, which is worth more than the pair until k has 96
+    k-blocks; the same bits in both forms."""
+    m, n = 2048, 2304
+    P = W.mx_problem(_capi.FMT_E4M3, m, n, k, True, seed=k, scale_lo=114, scale_hi=120)
+    A, B, SA, SB = (torch.from_numpy(x).cuda() for x in (P.A, P.B, P.SA, P.SB))
+    out = []
+    for form in (None, not pair):
+        D = torch.full((m, n), float("nan"), device="cuda")
+        op = c.GemmMx(STORAGE[P.fmt_a], STORAGE[P.fmt_b], pair=form)
+        st = op(op.Arguments(c.GemmCoord(m, n, k), c.MxTensorRef(A, SA, P.lda, P.ldsa), c.MxTensorRef(B, SB, P.ldb, P.ldsb),
+                             c.TensorRef(D, n), c.TensorRef(D, n), c.LinearCombination(1.0, 0.0)))
+        assert st == c.Status.kSuccess, _capi.last_error()
+        assert (_capi.last_plan().tile_n, _capi.last_plan().pair) == (256, pair if form is None else 1 - pair)
+        out.append(D)
+    assert torch.equal(out[0], out[1])
 
 
 @pytest.mark.parametrize("m,n,k,tile_n", [(512, 512, 512, 64), (1000, 900, 300, 64), (129, 65, 128, 64), (1024, 1216, 512, 128),
