@@ -58,7 +58,7 @@ struct Choice {
   int nacc = 2;
   int slices = 1;
   int stages = 4;
-  int piece_kb = 0;   // 8-bit MX: k-blocks summed in one accumulator (k_blocks: all)
+  int piece_kb = 0;   // MX: k-blocks summed in one accumulator (k_blocks: all)
 };
 
 int pick_bn_for_small(int nk) {
@@ -864,7 +864,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
       }
       return slices;
     };
-    // 8-bit MX: how many parts k would be cut into if every CTA had only an SM's share of HBM
+    // MX: how many parts k would be cut into if every CTA had only an SM's share of HBM
     // bandwidth to feed it.  The tensor cores lose low bits along a running sum, so this is
     // also how often a sum starts afresh: a launch with fewer slices than this keeps the
     // precision by summing in pieces (piece_kb), and one that cannot (BN > 64) keeps the slices.
@@ -891,7 +891,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
     if (d->split_k_slices > 1) {
       ch.slices = std::min(d->split_k_slices, k_blocks);
     } else {
-      const int parts = kind == kKindMxf8 && d->split_k_slices == 0 ? precision_parts(ch.BN) : 1;
+      const int parts = is_mx && d->split_k_slices == 0 ? precision_parts(ch.BN) : 1;
       const int piece_kb = parts > 1 ? std::max(1, k_blocks / parts) : ch.piece_kb;
       // a caller that asks for one of the two forms gets the same tile, slices and bits in either
       const bool form_given = (d->flags & (CPUOPS_B200_FLAG_PAIR_ON | CPUOPS_B200_FLAG_PAIR_OFF)) != 0;
@@ -1426,11 +1426,11 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
           epi_warps = 8;
       if (env_switches().epi_warps == 8 || env_switches().epi_warps == 4) epi_warps = env_switches().epi_warps;
     }
-    // 8-bit MX tiles with at most one 32-column chunk per epilogue warp may be summed in pieces,
+    // MX tiles with at most one 32-column chunk per epilogue warp may be summed in pieces,
     // added in f32 by those warps behind the MMAs (kPieces in gemm_kernel.cuh; wider tiles have
     // more accumulators than a warp has registers for).
     p.piece_kb = k_blocks;
-    if (kind == kKindMxf8 && !ch.pair && ch.BN <= 64 && ch.piece_kb < k_blocks) {
+    if (is_mx && !ch.pair && ch.BN <= 64 && ch.piece_kb < k_blocks) {
       epi_warps = 8;
       p.piece_kb = ch.piece_kb;
     }
@@ -1463,7 +1463,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
     const int64_t total_tiles = static_cast<int64_t>(p.m_tiles) * p.n_tiles * p.slices;
     unsigned grid = static_cast<unsigned>(std::min<int64_t>(total_tiles, sms));
     CUtensorMap tmSFA = tmA, tmSFB = tmA;  // used by the pair kernel's scale loads only
-    const GemmKernel kernel = gemm_kernel(kind, ch.pair, raw_scales);
+    const GemmKernel kernel = gemm_kernel(kind, ch.pair, raw_scales, p.piece_kb < k_blocks);
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3((epi_warps == 8 ? kGemmThreadsWide : kGemmThreads) + (raw_scales ? 32 * kScaleWriterWarps : 0));
     cfg.dynamicSmemBytes = static_cast<size_t>(smem);

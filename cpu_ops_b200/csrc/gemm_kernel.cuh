@@ -357,7 +357,15 @@ __device__ __forceinline__ void write_scale_atoms(const GemmParams& p, int write
 // tile instead of one in all, and a longer way from a free stage to a full one.  Re-laid-out /
 // raw: e4m3 512 x 2048 x 1024 12.8 / 8.8 us, 2048^3 17.9 / 15.4, 256 x 8192 x 8192 36.6 / 31.3; e2m1
 // 512 x 2048 x 1024 14.1 / 9.0, 1024 x 4096 x 4096 22.7 / 18.1, 2048 x 2304 x 8192 31.8 / 25.6.
-template <int KIND, bool kPair, bool kRaw = false>
+//
+// kPieces (MX, one CTA per tile, at most one 32-column chunk per epilogue warp): the accumulator is
+// taken down every p.piece_kb k-blocks and the pieces added by the epilogue warps.  The tensor
+// cores drop the low bits of a running sum: against float64, 8-bit results are off by 6e-10 per
+// element of k (2.4e-6 at k = 4096), e2m1 ones by 2.4e-10 once their scales span too many exponents
+// for f32 to hold the sums whole, and both by 2e-7 at any k in pieces of 256 elements.  An
+// instance of its own: as a run-time choice it cost the others up to 7 % (e2m1 2304 x 2304 x 8192 30.9 ->
+// 32.9 us, 512 x 2048 x 1024 7.2 -> 7.5).
+template <int KIND, bool kPair, bool kRaw = false, bool kPieces = false>
 __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWarps : 0), 1)
     gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                         const __grid_constant__ CUtensorMap tmB,
@@ -367,13 +375,9 @@ __global__ void __launch_bounds__(kGemmThreadsWide + (kRaw ? 32 * kScaleWriterWa
                         const __grid_constant__ CUtensorMap tmSFB, const GemmParams p) {
   constexpr bool kInt = (KIND == kKindI8);
   constexpr bool kMx = !kInt;
+  static_assert(!kPieces || (kMx && !kPair), "pieces: MX operands, one CTA per tile");
   static_assert(!kRaw || (kMx && !kPair), "raw scales: MX operands, one CTA per tile");
   constexpr int kCtas = kPair ? 2 : 1;
-  // 8-bit MX, one CTA per tile: the accumulator may be taken down every p.piece_kb k-blocks and
-  // the pieces added by the epilogue warps.  The tensor cores drop the low bits of a running
-  // sum: against float64, results are off by 6e-10 per element of k (2.4e-6 at k = 4096), and
-  // by 2e-7 at any k in pieces of 256 elements.
-  constexpr bool kPieces = KIND == kKindMxf8 && !kPair;
   // Programmatic dependent launch: the next kernel in the stream may become resident as
   // this one's CTAs retire; in return every role of this kernel that touches global memory
   // first waits for the kernel before it (griddepcontrol.wait), so stream order holds.

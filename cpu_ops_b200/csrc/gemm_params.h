@@ -67,7 +67,7 @@ struct GemmParams {
   int32_t BN;               // N tile (multiple of 32, <= 256)
   int32_t stages;           // smem pipeline depth
   int32_t nacc;             // TMEM accumulator buffers (1 or 2)
-  int32_t piece_kb;         // 8-bit MX, one CTA per tile: k-blocks summed in one accumulator
+  int32_t piece_kb;         // kPieces kernels: k-blocks summed in one accumulator
   int32_t raster_m;         // m-tiles per raster group (tile walk order)
   int32_t narrow_last;      // 1: the last tile column is computed at its own (narrower) width
   int32_t a_mn_major, b_mn_major;

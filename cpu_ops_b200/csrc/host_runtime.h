@@ -160,16 +160,18 @@ PreparedB* find_prepared(int device, const void* scales, int n, int k, int ld_sc
   return nullptr;
 }
 
-// The GEMM kernel's instantiations (raw scales: MX, no pairs).
+// The GEMM kernel's instantiations (raw scales and pieces of k: MX, no pairs).
 using GemmKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
-GemmKernel gemm_kernel(int kind, bool pair, bool raw_scales) {
+template <int KIND>
+GemmKernel gemm_mx_kernel(bool pair, bool raw_scales, bool pieces) {
+  if (pair) return gemm_tcgen05_kernel<KIND, true>;
+  if (raw_scales) return pieces ? gemm_tcgen05_kernel<KIND, false, true, true> : gemm_tcgen05_kernel<KIND, false, true>;
+  return pieces ? gemm_tcgen05_kernel<KIND, false, false, true> : gemm_tcgen05_kernel<KIND, false>;
+}
+GemmKernel gemm_kernel(int kind, bool pair, bool raw_scales, bool pieces) {
   if (kind == kKindI8) return pair ? gemm_tcgen05_kernel<kKindI8, true> : gemm_tcgen05_kernel<kKindI8, false>;
-  if (kind == kKindMxf8) {
-    if (raw_scales) return gemm_tcgen05_kernel<kKindMxf8, false, true>;
-    return pair ? gemm_tcgen05_kernel<kKindMxf8, true> : gemm_tcgen05_kernel<kKindMxf8, false>;
-  }
-  if (raw_scales) return gemm_tcgen05_kernel<kKindMxf4, false, true>;
-  return pair ? gemm_tcgen05_kernel<kKindMxf4, true> : gemm_tcgen05_kernel<kKindMxf4, false>;
+  return kind == kKindMxf8 ? gemm_mx_kernel<kKindMxf8>(pair, raw_scales, pieces)
+                           : gemm_mx_kernel<kKindMxf4>(pair, raw_scales, pieces);
 }
 
 // The decode kernel's.
@@ -273,8 +275,8 @@ int init_device(int device, DeviceState** out) {
         g_encode = reinterpret_cast<EncodeTiledFn>(fn);
       }
       for (int kind : {kKindI8, kKindMxf8, kKindMxf4})
-        for (int form = 0; form < 3; ++form)
-          CUDA_TRY(cudaFuncSetAttribute(gemm_kernel(kind, form == 1, form == 2),
+        for (int form = 0; form < 8; ++form)
+          CUDA_TRY(cudaFuncSetAttribute(gemm_kernel(kind, form & 1, form & 2, form & 4),
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, st.smem_optin));
       for (int kind : {kKindMxf8, kKindMxf4})
         for (bool pieces : {false, true})

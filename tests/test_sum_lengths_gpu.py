@@ -75,3 +75,14 @@ def test_decode_4_bit(gpu, m, n, k, longest):
     e = error(F4, m, n, k, -(-k // 512) * 16, 120, 134)
     assert _capi.last_plan().decode == 1
     assert e <= bound_e2m1(longest * 256), e
+
+
+# `longest`: k-blocks of 256 elements to a sum when k was cut by an SM's share of HBM bandwidth.
+@pytest.mark.parametrize("m,n,k,longest,lds_extra", [
+    (512, 512, 8192, 4, 0), (192, 320, 16384, 3, 0), (256, 512, 16384, 4, 1), (1024, 1024, 8192, 16, 0), (640, 1024, 32768, 32, 0),
+    (100, 60, 32768, 4, 0), (128, 128, 4096, 2, 0), (512, 1024, 16384, 13, 0)])
+def test_general_4_bit(gpu, m, n, k, longest, lds_extra):
+    """Scales over 15 exponents; scale rows that the kernel reads itself, and (an odd leading
+    dimension) ones that are re-laid-out."""
+    e = error(F4, m, n, k, k // 32 + lds_extra, 120, 134)
+    assert e <= bound_e2m1(longest * 256), e
