@@ -41,7 +41,7 @@ def build(force: bool = False, verbose: bool = False, instrument: bool = False) 
     if not force and not needs_build(out):
         return out
     cmd = ["nvcc", *NVCC_FLAGS, *(["-DCPUOPS_B200_INSTRUMENT"] if instrument else []),
-           *(["-Xptxas", "-v"] if verbose else []), "-o", str(out), *map(str, sources()), "-lcudart"]
+           *(["-Xptxas", "-v"] if verbose else []), "-o", str(out), *map(str, sources()), "-lcudart", "-ldl"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose:
         sys.stderr.write(res.stderr)

@@ -9,7 +9,12 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <dlfcn.h>
+#include <pthread.h>
+#include <signal.h>
+#if defined(__x86_64__)
 #include <immintrin.h>
+#endif
 
 #include <algorithm>
 #include <atomic>
@@ -21,6 +26,14 @@
 #include <thread>
 
 namespace {
+
+inline void spin_pause() {
+#if defined(__x86_64__)
+  _mm_pause();
+#elif defined(__aarch64__)
+  asm volatile("yield" ::: "memory");
+#endif
+}
 
 // `rows` rows of `width` bytes.
 struct RowCopy {
@@ -46,7 +59,9 @@ struct RowCopy {
 // scheduler's slice of 4 ms for it.  The threads are started by the first large copy of the
 // process, watch for the next copy for 200 us after each (a call's pieces follow one another
 // within microseconds), sleep otherwise, and end with the process (detached: nothing joins
-// them, in a forked child neither).  A caller that finds them busy with another caller's copy
+// them, in a forked child neither).  So that nobody else has to know of them, they take none of the
+// process's signals, and the shared library that holds their code is kept mapped when the
+// program closes it.  A caller that finds them busy with another caller's copy
 // does its own alone.
 class CopyThreads {
  public:
@@ -67,7 +82,7 @@ class CopyThreads {
     if (sleepers_.load() > 0) wake_.notify_all();
     while (take_part()) {
     }
-    while (done_.load(std::memory_order_acquire) < parts) _mm_pause();
+    while (done_.load(std::memory_order_acquire) < parts) spin_pause();
   }
 
  private:
@@ -92,6 +107,13 @@ class CopyThreads {
 
   void start() {
     started_ = true;
+    Dl_info self;
+    if (dladdr(reinterpret_cast<void*>(&spin_pause), &self) == 0 ||
+        dlopen(self.dli_fname, RTLD_NOW | RTLD_NOLOAD | RTLD_NODELETE) == nullptr)
+      return;  // (the callers copy alone)
+    sigset_t all, callers;
+    sigfillset(&all);
+    if (pthread_sigmask(SIG_SETMASK, &all, &callers) != 0) return;
     const unsigned cores = std::thread::hardware_concurrency();
     const int n = std::max(0, std::min(kThreads, static_cast<int>(cores) / 2 - 1));
     try {
@@ -99,6 +121,7 @@ class CopyThreads {
     } catch (...) {
       // no more threads to be had: the ones that exist share the work
     }
+    pthread_sigmask(SIG_SETMASK, &callers, nullptr);
   }
 
   void run() {
@@ -108,7 +131,7 @@ class CopyThreads {
       for (int i = 0; !found; ++i) {
         found = take_part();
         if (found) break;
-        _mm_pause();
+        spin_pause();
         if ((i & 63) == 63 && std::chrono::steady_clock::now() > until) break;
       }
       if (found) continue;

@@ -160,7 +160,10 @@ typedef struct cpuops_b200_gemm_desc {
  * provided the same call ran once on that stream before the capture began (the call
  * then finds its workspace in place; one that would have to allocate during capture
  * returns CPUOPS_B200_STATUS_INVALID_ARGUMENTS instead).  A workspace used under capture
- * is never freed, so graphs stay valid when later calls on the stream need more room. */
+ * is never freed, so graphs stay valid when later calls on the stream need more room.
+ * Large operands in pageable host memory are copied through 16 MB of pinned memory per
+ * device and by up to three threads besides the caller's, both kept until the process
+ * ends; the threads take no signals, and from then on the library cannot be unloaded. */
 CPUOPS_B200_API int cpuops_b200_gemm(const cpuops_b200_gemm_desc* desc);
 
 /* No counterpart in the reference.  u8 x s8 -> s32 GEMM through the two-stage
