@@ -173,10 +173,11 @@ struct DecodePlan {
 };
 
 // Clusters of `splits` CTAs of the decode kernel that can be resident at once (asked once per
-// device and size; a GPC's SMs are not a multiple of every size).
+// device, kind and size; a GPC's SMs are not a multiple of every size).  Both forms of the kernel
+// run one CTA per SM for their shared memory.
 int decode_clusters(DeviceState& st, int kind, int splits) {
-  int& known = st.decode_clusters[splits];
-  if (known < 0) {
+  int& known = st.decode_clusters[kind][splits];
+  if (known == 0) {
     cudaLaunchConfig_t probe = {};
     probe.gridDim = dim3(static_cast<unsigned>(splits * st.sm_count));
     probe.blockDim = dim3(kDecodeThreads);
@@ -194,9 +195,9 @@ int decode_clusters(DeviceState& st, int kind, int splits) {
       cudaGetLastError();
       n = 0;
     }
-    known = n;
+    known = n + 1;
   }
-  return known;
+  return known - 1;
 }
 
 // Grid, split and buffers of a decode launch: Mk weight rows (128-row tiles), Nk <= 64

@@ -119,8 +119,8 @@ struct DeviceState {
   // Largest number of two-CTA clusters of the pair kernel that can be resident at once,
   // per kind (-1: not asked yet; 0: cluster launch unavailable).
   int pair_clusters[3] = {-1, -1, -1};
-  // The same for the decode kernel's clusters, by cluster size.
-  int decode_clusters[kDecodeMaxSplits + 1] = {-1, -1, -1, -1, -1, -1, -1};
+  // The same for the decode kernel's clusters, by kind and cluster size (0: not asked yet, else one more).
+  int decode_clusters[3][kDecodeMaxSplits + 1] = {};
   TensorMapSlot tm_cache[kTensorMapSlots];
 };
 
