@@ -23,8 +23,7 @@ def test_pairs_in_one_wave(gpu, m, n, k, beta, pair):
     st = op(op.Arguments(c.GemmCoord(m, n, k), c.TensorRef(A, k), c.TensorRef(B, k), c.TensorRef(C, n),
                          c.TensorRef(D, n), c.LinearCombination(1, beta)))
     assert st == c.Status.kSuccess, _capi.last_error()
-    if _capi.last_plan().tile_n == 256:
-        assert _capi.last_plan().pair == pair
+    assert (_capi.last_plan().tile_n, _capi.last_plan().pair) == (256, pair)
     # |sums| < 2^53: exact in f64
     assert torch.equal(D, (A.double() @ B.double().T).to(torch.int32) + beta * C)
 

@@ -48,8 +48,9 @@ def test_same_bits(gpu, oracle, fmt, m, n, k, plan):
         check_mx(oracle, P, got[0][0].cpu().numpy(), 1.0, 0.5)
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][0], got[2][0])
     assert not torch.isnan(got[0][0]).any()
-    if m > 64 and not plan.get("pair") and (fmt == F4 or _capi.last_plan().slices == 1):
-        # (smaller ones take the decode kernel; pairs and 8-bit split k re-lay the scales out)
+    if m > 64 and not plan.get("pair"):
+        # (smaller ones take the decode kernel; pairs re-lay the scales out, as 8-bit launches with
+        # more work items than SMs over a long k do, of which there is none here)
         assert got[0][1] == got[1][1] == got[2][1] - 1, "the scales were not read by the GEMM kernel"
 
 
