@@ -943,7 +943,7 @@ static int gemm_body(const cpuops_b200_gemm_desc* d, int depth, int parent_piece
   }
 
   // ---- small-m MX problems take the decode kernel ---------------------------------------------
-  // (one launch, raw scales, every SM streaming an equal share of the weights).  It fetches the
+  // (one launch, raw scales, whole tiles per CTA or a tile's k cut over a cluster).  It fetches the
   // scale rows 16 bytes at a time, which wants 16-byte aligned bases and leading dimensions; a
   // forced tile width or slice count keeps the general kernel, whose plan those describe.
   DecodePlan dp;

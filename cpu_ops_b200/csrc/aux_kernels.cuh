@@ -142,8 +142,8 @@ __global__ void relayout_scales_kernel(const uint8_t* __restrict__ src0, uint8_t
 // A block reads 32 rows x kCols columns of every slab - kCols / 8 elements per thread, the words of several
 // slabs in flight - and turns them in shared memory where D's rows are contiguous.  Small outputs take
 // kCols = 8, many blocks: bound by the latency of those reads and by the gap between two launches, which
-// programmatic stream serialization hides: 192 x 320 x 16384 u8 x s8 in 22 slices, both kernels,
-// 13.5 -> 12.4 us.  Large ones take 32: with 8 a row of D is written 32 bytes at a time (GEMM and reduction,
+// programmatic stream serialization hides: 192 x 320 x 16384 u8 x s8, both kernels, 12.4 us in
+// 22 slices (13.5 without), 11.1 in 8.  Large ones take 32: with 8 a row of D is written 32 bytes at a time (GEMM and reduction,
 // kCols = 8 / 32: 640 x 1024 x 16384 in 3 slices 20.9 / 18.2 us, 1024 x 2048 x 16384 in 4 53.1 / 42.2,
 // 2048 x 2048 x 8192 in 2 76.7 / 55.7; 1000 x 300 x 8192 e4m3 in 8 20.9 / 22.5, too few blocks).
 template <bool kInt, int kCols>

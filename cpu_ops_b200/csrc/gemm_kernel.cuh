@@ -6,7 +6,7 @@
 // (block_gemm.h:119-150).
 //
 // Structure: persistent, warp-specialised, one CTA per SM, 224 threads (352 with
-// eight epilogue warps).
+// eight epilogue warps), and 128 more where the kernel reads raw scales (kRaw).
 //   warp 0 and the     TMA producers: A and B tiles (128-byte swizzled rows of
 //   last warp          k) and, for MX, the pre-arranged scale-factor chunks,
 //   (one lane each)    into a ring of shared-memory stages; the two take

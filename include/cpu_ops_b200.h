@@ -257,6 +257,8 @@ CPUOPS_B200_API int cpuops_b200_profile_collect(double* total_ms, int32_t* launc
  * until release_b: later cpuops_b200_gemm calls that pass the same b_scales / n / k /
  * ld_scales_b keep the tile-ordered copy of those scales that the tensor cores need
  * (built on the first such call, one per tile layout) instead of rebuilding it per call.
+ * A call with few tiles reads unregistered scales inside the GEMM kernel, with no launch in
+ * front; registered, it reads the kept copy of B's and re-lays A's out, which can take longer.
  * The caller must not modify the scale array while it is registered.  release_b
  * synchronises the device and frees the copies. */
 CPUOPS_B200_API int cpuops_b200_prepare_b(const cpuops_b200_gemm_desc* d, void** handle);

@@ -1,5 +1,5 @@
-"""The small-m MX kernel (one launch, raw scales read by TMA, every SM streaming an equal
-share of the weights, partial sums added in ascending k order) against the CPU oracle.
+"""The small-m MX kernel (one launch, raw scales read by the kernel, whole tiles per CTA or a tile's k
+cut over a cluster, partial sums added in ascending k order) against the CPU oracle.
 The reference has no kernel of its own for these shapes: its GEMV-like calls run the
 general blocked path (gemm/kernel/run_blocked.h:79-174), which the oracle restates."""
 import numpy as np
