@@ -48,5 +48,5 @@ def probe(tmp_path_factory):
 def test_threads_keep_to_themselves(probe):
     done = subprocess.run([sys.executable, "-c", PROGRAM, str(probe)], capture_output=True, text=True, timeout=60)
     assert done.returncode == 0, done.stderr
-    if (os.cpu_count() or 1) >= 4:
-        assert done.stdout.split() == ["helpers", str(min(3, (os.cpu_count() or 1) // 2 - 1))]
+    cores = len(os.sched_getaffinity(0))
+    assert done.stdout.split() == ["helpers", str(max(0, min(3, cores // 2 - 1)))]
